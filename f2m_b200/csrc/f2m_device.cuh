@@ -166,6 +166,107 @@ __device__ __forceinline__ void top3_insert(double x, double& v0, double& v1, do
     v1 = c0 ? v0 : (c1 ? x : v1);
     v0 = c0 ? x : v0;
 }
+// The two middle values a gradient needs (the 2nd and 3rd smallest) of a list
+// of three or four finite values, in either order: FP64 addition commutes, so
+// v1 + v2 is the same.  Three values take two compares and three selects, four
+// take four and six, where the insertion chain takes three and five for every
+// entry; most lists hold three or four entries (3.5-4.3 on average over a
+// solve).
+__device__ __forceinline__ void mid_of3(double a, double b, double c, double& p, double& q) {
+    const bool c1 = a < b;
+    const double mn = c1 ? a : b;
+    p = c1 ? b : a;
+    q = mn < c ? c : mn;
+}
+__device__ __forceinline__ void mid_of4(double a, double b, double c, double d, double& p, double& q) {
+    const bool c1 = a < b, c2 = c < d;
+    const double mn1 = c1 ? a : b, mx1 = c1 ? b : a;
+    const double mn2 = c2 ? c : d, mx2 = c2 ? d : c;
+    p = mn1 < mn2 ? mn2 : mn1;
+    q = mx1 < mx2 ? mx1 : mx2;
+}
+__device__ __forceinline__ double dmin2(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double dmax2(double a, double b) { return a < b ? b : a; }
+// the three smallest of four, sorted
+__device__ __forceinline__ void low3_of4(double a, double b, double c, double d, double& s0, double& s1, double& s2) {
+    const bool c1 = a < b, c2 = c < d;
+    const double mn1 = c1 ? a : b, mx1 = c1 ? b : a;
+    const double mn2 = c2 ? c : d, mx2 = c2 ? d : c;
+    const bool c3 = mn1 < mn2;
+    s0 = c3 ? mn1 : mn2;
+    const double t = c3 ? mn2 : mn1, u = mx1 < mx2 ? mx1 : mx2;
+    const bool c4 = t < u;
+    s1 = c4 ? t : u;
+    s2 = c4 ? u : t;
+}
+// v1 + v2 of a list of K values, 3 <= K <= 6 or K = 8 (+inf fills the places
+// past the list's end): selection networks, with the chain where the first
+// value or a selected one reaches its sentinels.
+template <int K>
+__device__ __forceinline__ double mid_sum(const double (&d)[K]) {
+    static_assert(K == 3 || K == 4 || K == 5 || K == 6 || K == 8, "");
+    double p, q;
+    if constexpr (K == 3) {
+        mid_of3(d[0], d[1], d[2], p, q);
+    } else if constexpr (K == 4) {
+        mid_of4(d[0], d[1], d[2], d[3], p, q);
+    } else {
+        double a0, a1, a2;
+        low3_of4(d[0], d[1], d[2], d[3], a0, a1, a2);
+        if constexpr (K == 5) {
+            p = dmin2(a1, dmax2(a0, d[4]));
+            q = dmin2(a2, dmax2(a1, d[4]));
+        } else if constexpr (K == 6) {
+            const bool c = d[4] < d[5];
+            const double b0 = c ? d[4] : d[5], b1 = c ? d[5] : d[4];
+            p = dmin2(dmin2(a1, b1), dmax2(a0, b0));
+            q = dmin2(a2, dmin2(dmax2(a1, b0), dmax2(a0, b1)));
+        } else {
+            double b0, b1, b2;
+            low3_of4(d[4], d[5], d[6], d[7], b0, b1, b2);
+            p = dmin2(dmin2(a1, b1), dmax2(a0, b0));
+            q = dmin2(dmin2(a2, b2), dmin2(dmax2(a1, b0), dmax2(a0, b1)));
+        }
+    }
+    double s = p + q;
+    if (!(d[0] < 1e6 && p < 1e6 && q < 1e6)) {
+        double x0 = d[0], x1 = 1e6, x2 = 1e6;
+#pragma unroll
+        for (int k = 1; k < K; ++k) {
+            if (d[k] < x0) { x2 = x1; x1 = x0; x0 = d[k]; }
+            else if (d[k] < x1) { x2 = x1; x1 = d[k]; }
+            else if (d[k] < x2) { x2 = d[k]; }
+        }
+        s = x1 + x2;
+    }
+    return s;
+}
+// Magnitudes at which the short forms above are the chain's: no NaN or
+// infinity can arise, and halving twice is exact (no subnormal), so a step
+// H + (-(v1 + v2) / 2) / 2 may be one fused multiply-add.
+__device__ __forceinline__ bool step_cost_plain(double D) { return D >= 1e-150 && D <= 1e150; }
+__device__ __forceinline__ bool step_pot_plain(double F) { return fabs(F) <= 1e150; }
+// Shared memory by 32-bit address (the step loops keep neighbour offsets in
+// registers).
+__device__ __forceinline__ double lds_f64(uint32_t a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_f64(uint32_t a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+// Reduced cost from D, the neighbour's and the own potential; `first`: the
+// neighbour is the lower id and is added first.
+__device__ __forceinline__ double red_of(double D, double hn, double hv, bool first) {
+    return (D + (first ? hn : hv)) + (first ? hv : hn);
+}
+
 // Reduced cost of position k of node v's list (the slot perm[r0 + k]).
 template <class HP>
 __device__ __forceinline__ double pdv(const Inst& I, int64_t r0, int k, int v, HP H, double hv) {

@@ -705,10 +705,11 @@ struct Team {
     long long* sredl;   // TEAM/32
     int* swarp;         // TEAM/32 + 1
     int* sint;          // 4 ints
+    // (ids 0-7; the step loop's barriers are 8-15)
     // barrier.sync without .aligned: a team may reach it with a diverged warp
     // (after `if (tid == 0) {...}`), which the aligned form (bar.sync) forbids
     __device__ __forceinline__ void sync() const {
-        asm volatile("barrier.sync %0, %1;" ::"r"(id + 1), "r"(TEAM) : "memory");
+        asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(TEAM) : "memory");
     }
     __device__ double max(double x) const {
         const int lane = tid & 31, w = tid >> 5;
@@ -791,10 +792,17 @@ struct Team {
 // memory in order; the rest live in the same layout in the instance's part of
 // a global arena (coalesced, L2-resident), and a slice that fits in neither
 // reads each node's list from the node-indexed copy.
+//
+// While the lists stand, the potentials are kept in slice order too (position
+// 32*s + l; the words hold positions): a lane's own potential is then read and
+// written with unit stride, where node order costs about six wavefronts for
+// each of the two.  The places past V in the last slice repeat its first node,
+// list included, so no lane is an exception.  Partitions and combs use node
+// order (to_nodes); an instance with a node-indexed slice stays in it.
 struct TeamMem {
     double* Ha;
     double* Hb;
-    uint16_t* ord;   // 32*NS: nodes in slice order
+    uint16_t* ord;   // 32*NS: nodes in slice order (the last slice is filled up with its first node)
     int* soff;       // NS: >= 0 shared offset; kSelGlobal + g: global offset g; kSelNode: node copy
     int* swid;       // NS: slice width (longest list)
     int* hist;       // 258: counting-sort buckets; hist[256] = total list length,
@@ -818,8 +826,8 @@ __device__ __forceinline__ TeamMem carve_team(unsigned char* base, size_t bytes,
     TeamMem M;
     M.NS = (V + 31) / 32;
     size_t o = 0;
-    M.Ha = reinterpret_cast<double*>(base + o); o += (size_t)V * 8;
-    M.Hb = reinterpret_cast<double*>(base + o); o = align16(o + (size_t)V * 8);
+    M.Ha = reinterpret_cast<double*>(base + o); o += (size_t)M.NS * 32 * 8;
+    M.Hb = reinterpret_cast<double*>(base + o); o += (size_t)M.NS * 32 * 8;
     M.soff = reinterpret_cast<int*>(base + o); o = align16(o + (size_t)M.NS * 4);
     M.swid = reinterpret_cast<int*>(base + o); o = align16(o + (size_t)M.NS * 4);
     M.hist = reinterpret_cast<int*>(base + o); o = align16(o + 258 * 4);
@@ -840,7 +848,7 @@ __device__ __forceinline__ TeamMem carve_team(unsigned char* base, size_t bytes,
 }
 __device__ __host__ inline size_t team_fixed_bytes(int V) {
     const int NS = (V + 31) / 32;
-    return (size_t)V * 16 + (size_t)NS * 8 + 258 * 4 + (size_t)NS * 64 + 5 * 16;
+    return (size_t)NS * 32 * 16 + (size_t)NS * 8 + 258 * 4 + (size_t)NS * 64 + 5 * 16;
 }
 
 __device__ __forceinline__ uint16_t ef_word(int v, int nbr) {
@@ -889,15 +897,248 @@ __device__ __forceinline__ void copy_ef_prefix(const Slot* __restrict__ ps, doub
     }
 }
 // one lane's column of a SELL-32 slice of width wdt from a node-indexed list
-// of n entries (padding: +inf, word 0)
+// of n entries (padding: +inf, word 0); pos maps node ids to positions (null:
+// the words keep node ids)
 __device__ __forceinline__ void fill_slice_lane(const double* __restrict__ gD, const uint16_t* __restrict__ gN,
-                                                int n, int wdt, double* __restrict__ dD, uint16_t* __restrict__ dW) {
+                                                const uint16_t* __restrict__ pos, int n, int wdt,
+                                                double* __restrict__ dD, uint16_t* __restrict__ dW) {
 #pragma unroll 4
     for (int k = 0; k < wdt; ++k) {
         const bool real = k < n;
         dD[32 * k] = real ? gD[k] : INFINITY;
-        dW[32 * k] = real ? gN[k] : (uint16_t)0;
+        uint16_t word = real ? gN[k] : (uint16_t)0;
+        if (real && pos) word = (uint16_t)(pos[word & 0x7fff] | (word & 0x8000));
+        dW[32 * k] = word;
     }
+}
+
+// What the step loops read: shared arrays by 32-bit address, the global part of
+// the slices by pointer.  Passed by value, so that the solver's own state need
+// not live in memory around the call.
+struct StepView {
+    uint32_t hc, hn;        // potentials in slice order, current and next
+    uint32_t eD, eW;        // SELL entries
+    uint32_t soff, swid;
+    const double* gsD;
+    const uint16_t* gsW;
+    int NS, warps, bar;     // slices, warps of the team, its step barrier
+};
+__device__ __forceinline__ int lds_i32(uint32_t a) {
+    int v;
+    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// One lane's list in a slice, in shared memory or in the global arena.
+struct ListSm {
+    uint32_t aD, aW;
+    __device__ __forceinline__ double D(int k) const { return lds_f64(aD + 256 * k); }
+    __device__ __forceinline__ uint32_t W(int k) const { return lds_u16(aW + 64 * k); }
+};
+struct ListGl {
+    const double* pD;
+    const uint16_t* pW;
+    __device__ __forceinline__ double D(int k) const { return pD[32 * k]; }
+    __device__ __forceinline__ uint32_t W(int k) const { return pW[32 * k]; }
+};
+__device__ __forceinline__ ListSm list_sm(const StepView& M, int off, int lane) {
+    return ListSm{M.eD + 8 * (off + lane), M.eW + 2 * (off + lane)};
+}
+__device__ __forceinline__ ListGl list_gl(const StepView& M, int off, int lane) {
+    return ListGl{M.gsD + (off - kSelGlobal) + lane, M.gsW + (off - kSelGlobal) + lane};
+}
+__device__ __forceinline__ void list_entry(const StepView& M, int off, int lane, int k, double& D, uint32_t& word) {
+    if (off >= 0) { const ListSm l = list_sm(M, off, lane); D = l.D(k); word = l.W(k); }
+    else { const ListGl l = list_gl(M, off, lane); D = l.D(k); word = l.W(k); }
+}
+// The potential after a step from the K entries of a slice of that width.  The
+// loads are issued before the first use.
+template <int K, class List>
+__device__ __forceinline__ double slice_step(const List& l, uint32_t hc, double hv) {
+    double D[K], x[K];
+    uint32_t word[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) { word[k] = l.W(k); D[k] = l.D(k); }
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = lds_f64(hc + 8 * (word[k] & 0x7fff));
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = red_of(D[k], x[k], hv, (word[k] & 0x8000) != 0);
+    return fma(mid_sum<K>(x), -0.25, hv);
+}
+// The same for a slice of any other width, out of line (the lists of the global
+// phase and a few later ones are longer).
+template <class List>
+__device__ __noinline__ double slice_step_wide(List l, int wd, uint32_t hc, double hv) {
+    if (wd == 4) return slice_step<4>(l, hc, hv);
+    if (wd == 5) return slice_step<5>(l, hc, hv);
+    if (wd == 6) return slice_step<6>(l, hc, hv);
+    return hv + half_grad(wd, [&](int k) {
+        const uint32_t word = l.W(k);
+        return red_of(l.D(k), lds_f64(hc + 8 * (word & 0x7fff)), hv, (word & 0x8000) != 0);
+    });
+}
+// the team's warps that have a slice (the others wait at the team barrier)
+__device__ __forceinline__ void step_barrier(int bar, int threads) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
+}
+
+// n Jacobi steps over fixed lists by warp w of the team, w < min(NS, warps),
+// whose slices are w, w + warps, ... (longest lists first).  A step is a short
+// dependent chain: a gather, two additions, the selection, a store and a
+// barrier.  On a full SM the shared-memory gathers bound it (a random 8-byte
+// gather takes about six wavefronts), so what does not change between
+// rebuilds -- D, the neighbours' offsets, the order flags and the own
+// potential, which only this lane writes -- stays in registers where it can.
+// A slice of three entries then takes 20 cycles of an SM; read from the SELL
+// arrays it takes about 35 in shared memory and 60 through L1 and L2.
+//
+// step_one: the warp's only slice, of width <= K, in registers.
+template <int K>
+__device__ __noinline__ void step_one(StepView M, int w, int lane, int n) {
+    const uint32_t own = 8u * (32 * w + lane);
+    uint32_t hc = M.hc, hn = M.hn;
+    const int bar = M.bar, threads = 32 * min(M.NS, M.warps);
+    const int wd = lds_i32(M.swid + 4 * w), off = lds_i32(M.soff + 4 * w);
+    double D[K], h = lds_f64(hc + own);
+    uint32_t a[K], first = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        uint32_t word = 0;
+        D[k] = INFINITY;
+        if (k < wd) list_entry(M, off, lane, k, D[k], word);
+        a[k] = 8u * (word & 0x7fff);
+        first |= (word >> 15) << k;
+    }
+    for (int it = 0; it < n; ++it) {
+        double x[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) x[k] = lds_f64(hc + a[k]);
+#pragma unroll
+        for (int k = 0; k < K; ++k) x[k] = red_of(D[k], x[k], h, (first >> k) & 1);
+        h = fma(mid_sum<K>(x), -0.25, h);
+        sts_f64(hn + own, h);
+        step_barrier(bar, threads);
+        const uint32_t t = hc; hc = hn; hn = t;
+    }
+}
+// step_slices: the last R slices, of width <= 3, in registers (16-bit byte
+// offsets, two to a register, so V <= 8,160), and with HEAD the first slice, of
+// width <= HEAD; with MEM the warp's other slices come from the SELL arrays.
+// (The few warps whose first slice is wider set the pace of a step: 96 slices
+// on 32 warps take 2,060 cycles when all are three wide, 4,020 with twelve
+// four-wide heads read from the SELL arrays.)
+constexpr int kPackedMaxV = 8160;
+template <int R, int HEAD, bool MEM>
+__device__ __noinline__ void step_slices(StepView M, int w, int lane, int n) {
+    uint32_t hc = M.hc, hn = M.hn;
+    const int bar = M.bar, threads = 32 * min(M.NS, M.warps), stride = M.warps;
+    const int nmem = MEM ? (M.NS - 1 - w) / stride + 1 - R : (HEAD ? 1 : 0);
+    constexpr int RR = R > 0 ? R : 1, HH = HEAD > 0 ? HEAD : 2;
+    double hD[HH], hh = 0.0;
+    uint32_t ha[HH / 2], hf = 0;
+    if (HEAD > 0) {
+        hh = lds_f64(hc + 8u * (32 * w + lane));
+        const int wd = lds_i32(M.swid + 4 * w), off = lds_i32(M.soff + 4 * w);
+#pragma unroll
+        for (int k = 0; k < HEAD; ++k) {
+            uint32_t word = 0;
+            hD[k] = INFINITY;
+            if (k < wd) list_entry(M, off, lane, k, hD[k], word);
+            const uint32_t o = 8u * (word & 0x7fff);
+            ha[k / 2] = (k & 1) ? (ha[k / 2] | o << 16) : o;
+            hf |= (word >> 15) << k;
+        }
+    }
+    double D[RR][3], h[RR];
+    uint32_t a01[RR], a2f[RR];  // offsets of the three neighbours, then the order flags
+    const uint32_t own0 = 8u * (32 * (w + nmem * stride) + lane);
+    if (R > 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int s = w + (nmem + r) * stride;
+            h[r] = lds_f64(hc + own0 + 256 * stride * r);
+            const int wd = lds_i32(M.swid + 4 * s), off = lds_i32(M.soff + 4 * s);
+            uint32_t a[3], first = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                uint32_t word = 0;
+                D[r][k] = INFINITY;
+                if (k < wd) list_entry(M, off, lane, k, D[r][k], word);
+                a[k] = 8u * (word & 0x7fff);
+                first |= (word >> 15) << k;
+            }
+            a01[r] = a[0] | a[1] << 16;
+            a2f[r] = a[2] | first << 16;
+        }
+    }
+    for (int it = 0; it < n; ++it) {
+        if (HEAD > 0) {
+            double x[HH];
+#pragma unroll
+            for (int k = 0; k < HEAD; ++k) x[k] = lds_f64(hc + ((k & 1) ? ha[k / 2] >> 16 : ha[k / 2] & 0xffff));
+#pragma unroll
+            for (int k = 0; k < HEAD; ++k) x[k] = red_of(hD[k], x[k], hh, (hf >> k) & 1);
+            if constexpr (HEAD > 0) hh = fma(mid_sum<HEAD>(x), -0.25, hh);
+        }
+        for (int s = w, j = 0; MEM && j < nmem; ++j, s += stride) {
+            const uint32_t own = 8u * (32 * s + lane);
+            const int wd = lds_i32(M.swid + 4 * s), off = lds_i32(M.soff + 4 * s);
+            const double hv = lds_f64(hc + own);
+            double x;
+            if (off >= 0) {
+                const ListSm l = list_sm(M, off, lane);
+                x = wd == 3 ? slice_step<3>(l, hc, hv) : slice_step_wide(l, wd, hc, hv);
+            } else {
+                const ListGl l = list_gl(M, off, lane);
+                x = wd == 3 ? slice_step<3>(l, hc, hv) : slice_step_wide(l, wd, hc, hv);
+            }
+            sts_f64(hn + own, x);
+        }
+        if (R > 0) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                double x[3];
+                x[0] = lds_f64(hc + (a01[r] & 0xffff));
+                x[1] = lds_f64(hc + (a01[r] >> 16));
+                x[2] = lds_f64(hc + (a2f[r] & 0xffff));
+#pragma unroll
+                for (int k = 0; k < 3; ++k) x[k] = red_of(D[r][k], x[k], h[r], (a2f[r] >> (16 + k)) & 1);
+                h[r] = fma(mid_sum<3>(x), -0.25, h[r]);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) sts_f64(hn + own0 + 256 * stride * r, h[r]);
+        }
+        if (HEAD > 0) sts_f64(hn + 8u * (32 * w + lane), hh);
+        step_barrier(bar, threads);
+        const uint32_t t = hc; hc = hn; hn = t;
+    }
+}
+template <int HEAD, bool MEM>
+__device__ __forceinline__ void step_slices_of(int R, const StepView& M, int w, int lane, int n) {
+    if (R == 1) step_slices<1, HEAD, MEM>(M, w, lane, n);
+    else if (R == 2) step_slices<2, HEAD, MEM>(M, w, lane, n);
+    else if (HEAD > 0 || R == 3) step_slices<3, HEAD, MEM>(M, w, lane, n);
+    else step_slices<4, 0, MEM>(M, w, lane, n);
+}
+// the loop for a warp's number of slices and their widths
+__device__ __noinline__ void run_steps(StepView M, int w, int lane, int n) {
+    const int nsl = (M.NS - 1 - w) / M.warps + 1;
+    const int w0 = lds_i32(M.swid + 4 * w);
+    if (nsl == 1 && w0 <= 8) {
+        if (w0 <= 3) step_one<3>(M, w, lane, n);
+        else if (w0 == 4) step_one<4>(M, w, lane, n);
+        else if (w0 <= 6) step_one<6>(M, w, lane, n);
+        else step_one<8>(M, w, lane, n);
+        return;
+    }
+    int R = 0;  // trailing slices of three entries
+    if (32 * M.NS <= kPackedMaxV)
+        while (R < min(nsl, 4) && lds_i32(M.swid + 4 * (w + (nsl - 1 - R) * M.warps)) <= 3) ++R;
+    if (R == nsl) step_slices_of<0, false>(R, M, w, lane, n);
+    else if (R == 0) step_slices<0, 0, true>(M, w, lane, n);
+    else if (R == nsl - 1 && R <= 3 && w0 <= 4) step_slices_of<4, false>(R, M, w, lane, n);
+    else if (R == nsl - 1 && R <= 3 && w0 <= 6) step_slices_of<6, false>(R, M, w, lane, n);
+    else if (R == nsl - 1 && R <= 3 && w0 <= 8) step_slices_of<8, false>(R, M, w, lane, n);
+    else step_slices_of<0, true>(R, M, w, lane, n);
 }
 
 template <int TEAM>
@@ -916,6 +1157,9 @@ struct Solver {
     long long wpad = 0;    // SELL entries the warps sweep (padding included), summed over iterations
     int checks = 0;
     bool capped = false;
+    bool plain = false;     // magnitudes allow the short step forms (step_cost_plain)
+    bool node_lists = false;  // some slice is read from the node-indexed copy
+    bool sliced = false;      // the potentials are in slice order
 
     __device__ Solver(const Batch& b, const DevParams& p, const Inst& i, const Team<TEAM>& t, TeamMem m)
         : B(b), P(p), I(i), T(t), M(m), Hc(m.Ha), Hn(m.Hb), row0(i.row[0]) {}
@@ -923,12 +1167,12 @@ struct Solver {
     __device__ int deg(int v) const { return (int)(I.row[v + 1] - I.row[v]); }
     __device__ void swap_f() { double* t = Hc; Hc = Hn; Hn = t; }
 
-    // grad/2 of the node in lane `lane` of slice s; v = that node (or -1)
-    __device__ __forceinline__ double slice_hgrad(int s, int lane, int& v, double& hv) const {
+    // grad/2 of the node v in lane `lane` of slice s; o: where its potential is
+    __device__ __forceinline__ double slice_hgrad(int s, int lane, int& v, int& o, double& hv) const {
         const int p = s * 32 + lane;
-        v = (p < I.V) ? (int)M.ord[p] : -1;
-        const int vv = v < 0 ? (int)M.ord[s * 32] : v;  // padding lanes shadow lane 0
-        hv = Hc[vv];
+        v = (int)M.ord[p];
+        o = sliced ? p : v;
+        hv = Hc[o];
         const int off = M.soff[s];
         if (off >= 0) {
             const double* Dp = M.eD + off + lane;
@@ -940,10 +1184,10 @@ struct Solver {
             const uint16_t* Wp = M.gsW + (off - kSelGlobal) + lane;
             return half_grad(M.swid[s], [&](int k) { return ef_d(Dp[32 * k], Wp[32 * k], hv, Hc); });
         }
-        const int64_t go = I.row[vv] - row0;
+        const int64_t go = I.row[v] - row0;
         const double* Dp = I.gD + go;
         const uint16_t* Wp = I.gN + go;
-        return half_grad(M.cnt[vv], [&](int k) { return ef_d(Dp[k], Wp[k], hv, Hc); });
+        return half_grad(M.cnt[v], [&](int k) { return ef_d(Dp[k], Wp[k], hv, Hc); });
     }
     // one Jacobi step: F += grad(F) (graph_cuda.cu:293-304), as H += grad/2;
     // frozen nodes keep F (block_EF_iter_BLOCK, graph_cuda.cu:278-289)
@@ -951,10 +1195,10 @@ struct Solver {
     __device__ __forceinline__ void step() {
         const int w = T.tid >> 5, lane = T.tid & 31;
         for (int s = w; s < M.NS; s += WARPS) {
-            int v;
+            int v, o;
             double hv;
-            const double g = slice_hgrad(s, lane, v, hv);
-            if (v >= 0) Hn[v] = (MASKED && B.shift[I.base + v] != 0.0) ? hv : hv + g;
+            const double g = slice_hgrad(s, lane, v, o, hv);
+            Hn[o] = (MASKED && B.shift[I.base + v] != 0.0) ? hv : hv + g;
         }
         wslots += M.hist[256];
         wpad += M.hist[257];
@@ -962,17 +1206,46 @@ struct Solver {
         swap_f();
         iters++;
     }
-    __device__ void jacobi() { step<false>(); }
     __device__ void jacobi_masked() { step<true>(); }
+
+    // n Jacobi steps (graph_cuda.cu:293-304)
+    __device__ void steps(int n) {
+        if (n <= 0) return;
+        if (!plain || !sliced) {
+            for (int it = 0; it < n; ++it) step<false>();
+            return;
+        }
+        const int w = T.tid >> 5;
+        if (w < min(M.NS, WARPS)) {
+            auto sh = [](const void* p) { return (uint32_t)__cvta_generic_to_shared(p); };
+            const StepView S{sh(Hc), sh(Hn), sh(M.eD), sh(M.eW), sh(M.soff), sh(M.swid),
+                             M.gsD, M.gsW, M.NS, WARPS, 8 + T.id};
+            run_steps(S, w, T.tid & 31, n);
+        }
+        T.sync();
+        wslots += (long long)n * M.hist[256];
+        wpad += (long long)n * M.hist[257];
+        iters += n;
+        if (n & 1) swap_f();
+    }
+    // whether the instance's costs and starting potentials allow the short step
+    // forms; F the potentials the descent starts from (null: 0), dF added to them
+    __device__ void check_plain(const double* F, const double* dF) {
+        bool ok = true;
+        for (int64_t a = row0 + T.tid; a < I.row[I.V]; a += TEAM) ok = ok && step_cost_plain(I.slot[a].D);
+        if (F)
+            for (int v = T.tid; v < I.V; v += TEAM)
+                ok = ok && step_pot_plain(F[I.base + v]) && (!dF || step_pot_plain(dF[I.base + v]));
+        plain = T.sum_ll(ok ? 0 : 1) == 0;
+    }
     // max |grad| (max_node_grad, graph_cuda_maxmin.hpp:29-37)
     __device__ double grad_max() const {
         const int w = T.tid >> 5, lane = T.tid & 31;
         double m = 0.0;
         for (int s = w; s < M.NS; s += WARPS) {
-            int v;
+            int v, o;
             double hv;
-            const double g = slice_hgrad(s, lane, v, hv);
-            if (v >= 0) m = fmax(m, fabs(g));
+            m = fmax(m, fabs(slice_hgrad(s, lane, v, o, hv)));
         }
         return 2.0 * T.max(m);
     }
@@ -1030,6 +1303,9 @@ struct Solver {
             if (key >= 0) M.ord[base + __popc(peers & ((1u << lane_) - 1u))] = (uint16_t)v;
         }
         T.sync();
+        if (V + T.tid < 32 * M.NS) M.ord[V + T.tid] = M.ord[32 * (M.NS - 1)];  // (fewer than 32 places)
+        uint16_t* pos = reinterpret_cast<uint16_t*>(Hn);  // position of each node; Hn is free here
+        for (int p = T.tid; p < V; p += TEAM) pos[M.ord[p]] = (uint16_t)p;
         // slice widths (longest list of the slice) and offsets in the cache
         const int w = T.tid >> 5, lane = T.tid & 31;
         for (int s = w; s < M.NS; s += WARPS) {
@@ -1056,6 +1332,7 @@ struct Solver {
         }
         if (T.tid == 0) M.hist[257] = carry;  // read after the barriers below
         lead = T.max_ll(lead);
+        node_lists = carry - lead > M.gcap;
         for (int s = T.tid; s < M.NS; s += TEAM) {
             const int pos = M.soff[s], size = 32 * M.swid[s];
             if (pos + size <= M.cap) continue;
@@ -1069,13 +1346,24 @@ struct Solver {
             if (off == kSelNode) continue;
             double* dD = (off >= 0) ? M.eD + off : M.gsD + (off - kSelGlobal);
             uint16_t* dW = (off >= 0) ? M.eW + off : M.gsW + (off - kSelGlobal);
-            const int p = s * 32 + lane;
-            const int v = (p < V) ? (int)M.ord[p] : -1;
-            const int n = (v >= 0) ? M.cnt[v] : 0;
-            const int64_t go = (v >= 0) ? I.row[v] - row0 : 0;
-            fill_slice_lane(I.gD + go, I.gN + go, n, M.swid[s], dD + lane, dW + lane);
+            const int v = (int)M.ord[s * 32 + lane];
+            const int64_t go = I.row[v] - row0;
+            fill_slice_lane(I.gD + go, I.gN + go, node_lists ? nullptr : pos, M.cnt[v], M.swid[s], dD + lane, dW + lane);
         }
         T.sync();
+        if (node_lists) return;
+        for (int p = T.tid; p < 32 * M.NS; p += TEAM) Hn[p] = Hc[M.ord[p]];
+        T.sync();
+        swap_f();
+        sliced = true;
+    }
+    // the potentials back in node order (before partitions and combs)
+    __device__ void to_nodes() {
+        if (!sliced) return;
+        for (int p = T.tid; p < I.V; p += TEAM) Hn[M.ord[p]] = Hc[p];
+        T.sync();
+        swap_f();
+        sliced = false;
     }
     __device__ void finish_partition() {
         T.sync();
@@ -1083,6 +1371,7 @@ struct Solver {
     }
     // check_OPT + update_EF (graph_cuda.cu:229-271) with cuda_partition_v2
     __device__ double check_opt() {
+        to_nodes();
         for (int v = T.tid; v < I.V; v += TEAM) {
             const int d = deg(v);
             M.cnt[v] = (d < P.ef_small_deg) ? d : qpart_ef_pair(I, I.row[v], v, Hc, d, P.ef_thr, P.ef_min);
@@ -1095,21 +1384,15 @@ struct Solver {
     // max |grad| was taken over the same potentials and active sets, so that
     // value is the entry gradient MA.
     __device__ void block_ef(int N, double MA) {
-        int count_M = 0;
-        for (int it = 0; it < N; ++it) {
-            jacobi();
-            if (++count_M >= P.check_every) {
-                if (MA < P.error_B) break;
-                count_M = 0;
-            }
-        }
+        steps(MA < P.error_B ? min(N, max(P.check_every, 1)) : N);
     }
     // block_GLOB (graph_cuda.cu:363-430)
     __device__ void block_glob() {
         for (int v = T.tid; v < I.V; v += TEAM) M.cnt[v] = min(deg(v), P.glob_K);  // setvalue2V
         finish_partition();
         for (int go = 0; go < P.glob_rounds; ++go) {
-            for (int it = 0; it < P.glob_inner; ++it) jacobi();
+            steps(P.glob_inner);
+            to_nodes();
             // cuda_partition_v4 (graph_cuda_partition.hpp:89-115)
             for (int v = T.tid; v < I.V; v += TEAM) {
                 const int d = deg(v);
@@ -1152,6 +1435,7 @@ struct Solver {
     // Comb extraction (graph_cuda_comb.hpp:415-475), the device comb check and
     // the primal; writes the per-node state for the host and the results.
     __device__ void combs_and_primal(int b, double M_, bool accumulate) {
+        to_nodes();
         const int V = I.V;
         const double porog = P.porog;
         int* ccnt = reinterpret_cast<int*>(Hn);  // Hn is free: room for 2V ints
@@ -1301,14 +1585,14 @@ __global__ void __launch_bounds__(TEAM* TEAMS) k_solve(Batch B, DevParams P, con
             // (resuming from given potentials skips the global phase: run_fix,
             // the schedule the reference runs after a repair shift)
             for (int v = T.tid; v < I.V; v += TEAM) M.Ha[v] = B.F0 ? 0.5 * B.F0[I.base + v] : 0.0;
-            T.sync();
+            S.check_plain(B.F0, nullptr);
             Mg = B.F0 ? S.run_fix() : S.run_start();
         } else {
             // cuda_IRREGULAR_B_recompute (graph_cuda_comb.hpp:542-574): shift the
             // potentials of irregular combs, 20 frozen iterations, run_fix; the
             // EF lists of the last update_EF are in the node-indexed copy
             for (int v = T.tid; v < I.V; v += TEAM) M.Ha[v] = 0.5 * (B.F[I.base + v] + B.shift[I.base + v]);
-            T.sync();
+            S.check_plain(B.F, B.shift);
             S.rebuild_ef(false);
             for (int go = 0; go < P.frozen_iters; ++go) S.jacobi_masked();
             Mg = S.run_fix();

@@ -1,0 +1,49 @@
+"""The step loops of the team solver hold a warp's slices in registers where
+they fit and read the rest from the SELL arrays; which loop runs follows from
+the instance's size, the team's width and the list lengths.  The potentials
+must equal the oracle's bit for bit in every one of them."""
+import numpy as np
+import pytest
+
+import f2m_b200
+from f2m_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 129, 1025, 2049, 4097, 8161, 8200])
+def test_potentials_at_slice_edges(ctx, oracle, n):
+    """Around whole slices, one slice a warp, four slices a warp, and the last
+    size whose offsets fit 16 bits (8,160)."""
+    x, y = synth.uniform_int_points(n, 500 + n)
+    o = oracle.solve_points(x, y, 12, threads=8)
+    r = ctx.solve_points(x, y, 12)
+    assert r.status == o.status
+    assert np.array_equal(r.F, o.F)
+
+
+@pytest.mark.parametrize("bounds", [[4, 5, 6], [4, 5, 3000], [4, 2500, 4000], [700, 2000, 5000]])
+def test_potentials_do_not_depend_on_the_team(ctx, oracle, bounds):
+    """One to eight slices a warp, with four- to eight-entry and
+    longer first slices (the lattice's lists)."""
+    start = f2m_b200.get_class_bounds()
+    try:
+        f2m_b200.set_class_bounds(bounds)
+        for (x, y), N in [(synth.uniform_int_points(2000, 9), 16), (synth.lattice_points(700, 5, keep=0.3), 10)]:
+            o = oracle.solve_points(x, y, N)
+            r = ctx.solve_points(x, y, N)
+            assert r.status == o.status
+            assert np.array_equal(r.F, o.F)
+    finally:
+        f2m_b200.set_class_bounds(start)
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -600, 2.0 ** -400, 1.0])
+def test_costs_outside_the_short_forms_range(ctx, oracle, scale):
+    """Costs below 1e-150 take the reference's chain step by step."""
+    x, y = synth.uniform_int_points(300, 17)
+    g = oracle.build_graph(x, y, 10)
+    o = oracle.solve_graph(g.n_nodes, g.v1, g.v2, g.D * scale, g.Do, label=g.label)
+    r = ctx.solve_graph(g.n_nodes, g.v1, g.v2, g.D * scale, g.Do, labels=g.label)
+    assert r.status == o.status
+    assert np.array_equal(r.F, o.F)
