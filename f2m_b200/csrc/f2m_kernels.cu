@@ -1763,10 +1763,26 @@ void solve_get_bounds(int32_t* max_n) {
 
 int32_t solve_max_nodes() { return 10000; }
 int solve_num_classes() { return kNumClasses; }
-int solve_class_of(int32_t n) {
+// The narrowest class for a call of n_inst instances: the widest one whose
+// teams are all resident at once.  The size bounds are for throughput, a full
+// GPU; a call with fewer instances than that leaves SMs idle, and a solve is
+// thousands of dependent steps, so each instance then gets the most threads it
+// can have: a call of up to 148 instances runs on 1,024-thread teams, one to an
+// SM (64 instances of 50-320 points 8.7 -> 4.4 ms with it, one of 300 points
+// 3.4 -> 2.6 ms, against the 128-thread teams their size asks for).
+int solve_wide_class(int64_t n_inst) {
+    int dev = 0, sms = 0, wide = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     for (int c = 0; c < kNumClasses; ++c)
-        if (n <= kClasses[c].max_n) return c;
-    return kNumClasses - 1;
+        if (n_inst <= (int64_t)sms * kClasses[c].teams) wide = c;
+    return wide;
+}
+// class of an instance of n points in a call whose narrowest class is `wide`
+int solve_class_of(int32_t n, int wide) {
+    int c = 0;
+    while (c < kNumClasses - 1 && n > kClasses[c].max_n) ++c;
+    return std::max(c, wide);
 }
 
 // Shared memory of the solver CTAs.  A CTA does not take the whole opt-in

@@ -189,9 +189,10 @@ void make_plan(Plan& pl, int32_t n_inst, const int64_t* offs, int32_t N) {
     pl.seg.assign(nc, 0);
     pl.cnt.assign(nc, 0);
     pl.class_vcap.assign(nc, 4);
+    const int wide = solve_wide_class(n_inst);
     for (int32_t b = 0; b < n_inst; ++b) {
         const int32_t n = (int32_t)(offs[b + 1] - offs[b]);
-        const int c = solve_class_of(n);
+        const int c = solve_class_of(n, wide);
         pl.cnt[c]++;
         pl.class_vcap[c] = std::max(pl.class_vcap[c], n);
     }
@@ -1033,7 +1034,7 @@ f2m_status complete_instance(f2m_ctx* ctx, DevCall& C, int b, const f2m_params& 
                 (e = cudaMemcpyAsync(C.ord, &one, sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(B.status + b, &st, sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
                 (e = (C.grid ? launch_solve_grid(B, to_dev(prm), C.G, b, H.V, true, ctx->stream, &ctx->launches)
-                             : launch_refit_class(solve_class_of(H.V), B, to_dev(prm), C.ord, 1, B.queue + 7,
+                             : launch_refit_class(solve_class_of(H.V, solve_wide_class(1)), B, to_dev(prm), C.ord, 1, B.queue + 7,
                                                   std::max<int32_t>(H.V, 4), ctx->stream, &ctx->launches))) != cudaSuccess ||
                 (e = cudaMemcpyAsync(H.F.data(), B.F + ibase, H.V * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(H.efcnt.data(), B.efcnt + ibase, H.V * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
@@ -2407,7 +2408,7 @@ f2m_status f2m_solve_file(f2m_ctx* ctx, const char* path, int32_t top_k, const f
         // the host-assembled graph may have fewer nodes than points: re-plan
         // the class from the node count
         std::vector<int32_t> one{0};
-        const int c = solve_class_of(H.V);
+        const int c = solve_class_of(H.V, solve_wide_class(1));
         F2M_CUDA(cudaMemcpyAsync(C.ord, one.data(), sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
         F2M_CUDA(launch_solve_class(c, C.B, to_dev(prm), C.ord, 1, C.B.queue + 6,
                                     std::max<int32_t>(H.V, 4), ctx->stream, &ctx->launches));
@@ -2575,7 +2576,7 @@ extern "C" f2m_status f2m_solve_points_noalloc(const double* d_x, const double* 
     if (cudaGetLastError() != cudaSuccess) return F2M_ERR_CUDA;
     if (launch_prep(B, s, &launches) != cudaSuccess || launch_knn(B, scan, s, &launches) != cudaSuccess ||
         launch_graph(B, deg, scan, s, &launches) != cudaSuccess ||
-        launch_solve_class(solve_class_of(n), B, to_dev(prm), ord, 1, B.queue, std::max<int32_t>(n, 4), s,
+        launch_solve_class(solve_class_of(n, solve_wide_class(1)), B, to_dev(prm), ord, 1, B.queue, std::max<int32_t>(n, 4), s,
                            &launches) != cudaSuccess ||
         launch_axb(B, to_dev(prm), s, &launches) != cudaSuccess)
         return F2M_ERR_CUDA;
