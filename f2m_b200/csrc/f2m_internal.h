@@ -241,7 +241,17 @@ struct SmoothBatch {
     int32_t* nbr = nullptr;             // [S]
     int64_t* mirror = nullptr;          // [S] slot of the same edge in the neighbour's list
     float* c = nullptr;                 // [S]
-    double tau = 0, omega = 0;
+    int32_t W = 0;                      // columns of a slice (0: per-step path, no slices)
+    int64_t n_warps = 0;                // slices, or warps of the per-step kernels (whole ones per instance)
+    const int64_t* sbase = nullptr;     // [n_inst + 1] first of them of each instance
+    const int32_t* order = nullptr;     // [n_inst] instances, largest first
+    int64_t s_cap = 0;                  // entries of the [S] arrays
+    uint2* sent = nullptr;              // [S] each list by ascending cost: cost bits, local neighbour
+    int32_t* splace = nullptr;          // [S] place of that entry in the CSR row
+    double* gs = nullptr;               // [S] the steps' share of dL/dc, in that order
+    uint2* sell = nullptr;              // [n_warps * 32 * W] the first entries of each list in slices of 32 lanes
+    double* gsell = nullptr;            // [n_warps * 32 * W] their share of dL/dc
+    double tau = 0, inv_tau = 0, omega = 0;
     int32_t iters = 0, newton_max = 0, ckpt = 1, n_ck = 1;
     double* L = nullptr;                // [n_inst]
     const double* dL = nullptr;         // [n_inst] upstream gradient
@@ -254,7 +264,10 @@ struct SmoothBatch {
     double* segs = nullptr;             // [n_total * ckpt] their roots
     double* lam = nullptr;              // [n_total]
     double* lam2 = nullptr;             // [n_total]
-    double* q = nullptr;                // [S]
+    double* mu = nullptr;               // [n_total] omega lam / D of the step being reversed
+    double* segt = nullptr;             // [n_total * ckpt] reach bounds of the recomputed roots
+    double* segm = nullptr;             // [n_inst * ckpt] largest potential of each recomputed iterate
+    long long* umax = nullptr;          // [(3 iters + 4) * n_inst] per-instance maxima (per-step path)
     double* gc = nullptr;               // [S] dL/dc accumulated per slot
     float* gx = nullptr;                // [n_total]
     float* gy = nullptr;                // [n_total]
@@ -267,6 +280,7 @@ cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaSt
                                 int64_t* launches);
 cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches);
 int32_t smooth_max_nodes();
+int smooth_nodes_per_warp(bool steps, int64_t n_total);
 // Rate probe of the smoothed bound's logistic term (one exp and two
 // divisions, the Newton sums' unit of work), and its work per launch.
 cudaError_t launch_logit_probe(int blocks, int iters, double* out, cudaStream_t s);

@@ -1918,7 +1918,7 @@ cudaError_t smooth_steps_graph(f2m_ctx* ctx, SmoothBatch& B, bool grad) {
     int64_t tb, ob;
     std::memcpy(&tb, &B.tau, 8);
     std::memcpy(&ob, &B.omega, 8);
-    const std::vector<int64_t> key{B.n_total, B.n_inst, B.N, B.iters, B.ckpt, B.newton_max, grad ? 1 : 0,
+    const std::vector<int64_t> key{B.n_total, B.n_inst, B.n_warps, B.N, B.iters, B.ckpt, B.newton_max, grad ? 1 : 0,
                                    tb, ob, (int64_t)(intptr_t)ctx->dev, (int64_t)ctx->dev_cap};
     if (ctx->sgraph && key == ctx->skey) {
         ctx->launches += ctx->sgraph_launches;
@@ -1989,7 +1989,23 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     const int32_t K = sp.checkpoint;
     const int32_t nck = std::max(1, (sp.iters + K - 1) / K);
     const int64_t S = 2 * n * N + 8 * n;  // union lists: own N + reverse (+ slack)
-    const bool steps = sp.solver == 2 || (sp.solver == 0 && n_inst < ctx->sms);
+    // Under two instances an SM a pass of one CTA waits on its own latency and
+    // the whole GPU takes each pass instead: 200 instances of 200-1,200 points
+    // 15.1 ms (one CTA each) / 15.7 ms (a launch a pass) at tau 1e-3, 80 / 27 at
+    // 5e-2; 500 of 200-2,000 points 29 / 59 and 138 / 96.
+    const bool steps = sp.solver == 2 || (sp.solver == 0 && n_inst < 2 * ctx->sms);
+    std::vector<int64_t> sbase(n_inst + 1, 0);  // slices, or warps of the per-step kernels
+    const int64_t npw = smooth_nodes_per_warp(steps, n);
+    std::vector<int32_t> order(n_inst);
+    for (int32_t b = 0; b < n_inst; ++b) {
+        sbase[b + 1] = sbase[b] + (offs[b + 1] - offs[b] + npw - 1) / npw;
+        order[b] = b;
+    }
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int32_t a, int32_t b) { return offs[a + 1] - offs[a] > offs[b + 1] - offs[b]; });
+    const int64_t n_warps = sbase[n_inst];
+    // slices hold 2 N entries of a node, nearly every list
+    const int32_t W = steps ? 0 : (int32_t)((2 * (int64_t)N * npw + 31) / 32);
     SmoothBatch B;
     int64_t* scan = nullptr;
     double* dLd = nullptr;
@@ -2008,6 +2024,11 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
         B.nbr = A.take<int32_t>(S);
         B.mirror = A.take<int64_t>(S);
         B.c = A.take<float>(S);
+        B.sbase = A.take<int64_t>(n_inst + 1);
+        B.order = A.take<int32_t>(n_inst);
+        B.sent = A.take<uint2>(S);
+        B.splace = A.take<int32_t>(S);
+        if (!steps) B.sell = A.take<uint2>(n_warps * 32 * W);
         B.L = A.take<double>(n_inst);
         dLd = A.take<double>(n_inst);
         B.queue = A.take<int32_t>(1);
@@ -2016,6 +2037,7 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
             B.ua = A.take<double>(n);
             B.ub = A.take<double>(n);
             B.Lp = A.take<double>(n);
+            B.umax = A.take<long long>((3 * (int64_t)sp.iters + 4) * n_inst);
         }
         if (grad) {
             B.ck = A.take<double>(n * nck);
@@ -2023,7 +2045,11 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
             B.segs = A.take<double>(n * K);
             B.lam = A.take<double>(n);
             B.lam2 = A.take<double>(n);
-            B.q = A.take<double>(S);
+            B.mu = A.take<double>(n);
+            B.segt = A.take<double>(n * K);
+            B.segm = A.take<double>((int64_t)n_inst * K);
+            B.gs = A.take<double>(S);
+            if (!steps) B.gsell = A.take<double>(n_warps * 32 * W);
             B.gc = A.take<double>(S);
             B.gx = A.take<float>(n);
             B.gy = A.take<float>(n);
@@ -2039,7 +2065,11 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     B.n_inst = n_inst;
     B.N = N;
     B.n_total = n;
+    B.W = W;
+    B.n_warps = n_warps;
+    B.s_cap = S;
     B.tau = sp.tau;
+    B.inv_tau = 1.0 / sp.tau;
     B.omega = sp.damping;
     B.iters = sp.iters;
     B.newton_max = sp.newton_max;
@@ -2053,6 +2083,10 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     F2M_CUDA(cudaMemcpyAsync(const_cast<float*>(B.x), x, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<float*>(B.y), y, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(dLd, up.data(), n_inst * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(B.sbase), sbase.data(), (n_inst + 1) * sizeof(int64_t),
+                             cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(B.order), order.data(), n_inst * sizeof(int32_t),
+                             cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(launch_smooth_graph(B, scan, ctx->stream, &ctx->launches));
     B.solver = steps ? 2 : 1;
     ctx->smooth_terms = -1;

@@ -19,6 +19,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "f2m_device.cuh"
 #include "f2m_internal.h"
 
@@ -41,12 +43,42 @@ __device__ __forceinline__ int find_inst(const int64_t* offs, int n_inst, int64_
 }
 
 /* ---------------- kNN: warp per point, brute force over its instance ---- */
-// Each warp keeps the point's best N keys (cost bits << 32 | local index; the
-// cost is non-negative, so the unsigned order is (cost, index)) as a sorted
-// list spread over two registers per lane (elements l and 32 + l).
+// Sorts 64 keys ascending, elements l (a) and 32 + l (b) in lane l.
+template <class T>
+__device__ __forceinline__ void warp_sort64(T& a, T& b) {
+    const int l = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 64; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j == 32) {
+                if (b < a) { const T t = a; a = b; b = t; }
+            } else {
+                const T pa = __shfl_xor_sync(0xffffffffu, a, j), pb = __shfl_xor_sync(0xffffffffu, b, j);
+                const bool low = (l & j) == 0;
+                // (element 32 + l differs from l in bit 5 only, which decides the direction at k = 32)
+                const bool ua = (l & k) == 0 || k == 64, ub = k == 32 ? false : ua;
+                a = ((low == ua) == (pa < a)) ? pa : a;
+                b = ((low == ub) == (pb < b)) ? pb : b;
+            }
+        }
+    }
+}
+// Each warp finds its point's N smallest keys (cost bits << 32 | local index;
+// the cost is non-negative, so the unsigned order is (cost, index)).
+//
+// N <= 32: a first scan keeps the two smallest costs of every lane; the N-th
+// smallest of those 64 bounds the N-th smallest cost (a few ranks above it,
+// as a lane seldom holds three of the first N), and a second scan collects
+// what lies at or below it -- one sort instead of an insertion for each of the
+// N ln(V / N) improvements (19 ms of insertions for 1,024 instances of 1,100
+// points on average, N = 24).  More than 64 collected (ties), or fewer than N
+// (NaN), take the insertion, as N > 32 does.
+constexpr int kKnnBuf = 64;
 __global__ void __launch_bounds__(256) k_sknn(SmoothBatch S) {
-    const int lane = threadIdx.x & 31;
-    const int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    __shared__ unsigned long long s_key[8][kKnnBuf];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t g = (int64_t)blockIdx.x * 8 + wid;
     if (g >= S.n_total) return;
     const int b = find_inst(S.offs, S.n_inst, g);
     const int64_t base = S.offs[b];
@@ -54,13 +86,45 @@ __global__ void __launch_bounds__(256) k_sknn(SmoothBatch S) {
     const int N = min(S.N, V - 1);
     const int i = (int)(g - base);
     const float xi = S.x[g], yi = S.y[g];
+    const float* px = S.x + base;
+    const float* py = S.y + base;
     unsigned long long A = ~0ull, Bk = ~0ull;
+    bool insert = N > 32;
+    if (!insert) {
+        float m0 = INFINITY, m1 = INFINITY;
+#pragma unroll 4
+        for (int j = lane; j < V; j += 32) {
+            const float c = j != i ? sdist(xi, yi, px[j], py[j]) : INFINITY;
+            m1 = fminf(m1, fmaxf(m0, c));
+            m0 = fminf(m0, c);
+        }
+        warp_sort64(m0, m1);
+        const float bound = __shfl_sync(0xffffffffu, m0, N - 1);
+        int cnt = 0;
+        for (int j0 = 0; j0 < V; j0 += 32) {
+            const int j = j0 + lane;
+            const float c = j < V && j != i ? sdist(xi, yi, px[j], py[j]) : NAN;
+            const unsigned m = __ballot_sync(0xffffffffu, c <= bound);
+            const int at = cnt + __popc(m & ((1u << lane) - 1u));
+            if (c <= bound && at < kKnnBuf) s_key[wid][at] = ((unsigned long long)__float_as_uint(c) << 32) | (unsigned)j;
+            cnt += __popc(m);
+        }
+        __syncwarp();
+        insert = cnt < N || cnt > kKnnBuf;
+        if (!insert) {
+            A = lane < cnt ? s_key[wid][lane] : ~0ull;
+            Bk = 32 + lane < cnt ? s_key[wid][32 + lane] : ~0ull;
+            warp_sort64(A, Bk);
+        }
+    }
+    // insertion into a sorted list spread over two registers per lane
+    // (elements l and 32 + l)
     unsigned long long thr = ~0ull;  // element N-1
-    for (int j0 = 0; j0 < V; j0 += 32) {
+    for (int j0 = 0; insert && j0 < V; j0 += 32) {
         const int j = j0 + lane;
         unsigned long long key = ~0ull;
         if (j < V && j != i) {
-            const float c = sdist(xi, yi, S.x[base + j], S.y[base + j]);
+            const float c = sdist(xi, yi, px[j], py[j]);
             key = ((unsigned long long)__float_as_uint(c) << 32) | (unsigned)j;
         }
         unsigned m = __ballot_sync(0xffffffffu, key < thr);
@@ -127,15 +191,32 @@ __global__ void k_ssort(SmoothBatch S) {
     if (g >= S.n_total) return;
     int32_t* a = S.tnbr + S.tcap[g];
     const int n = S.N + S.rdeg[g];
-    for (int i = 1; i < n; ++i) {
-        const int32_t v = a[i];
-        int j = i - 1;
-        while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-        a[j + 1] = v;
-    }
+    auto sort = [n](int32_t* out, const int32_t* in) {
+        for (int i = 0; i < n; ++i) {
+            const int32_t v = in[i];
+            int j = i - 1;
+            while (j >= 0 && out[j] > v) { out[j + 1] = out[j]; --j; }
+            out[j + 1] = v;
+        }
+    };
     int m = 0;
-    for (int i = 0; i < n; ++i)
-        if (a[i] >= 0 && (m == 0 || a[m - 1] != a[i])) a[m++] = a[i];
+    auto pack = [&](const int32_t* in) {
+        int32_t last = -1;
+        for (int i = 0; i < n; ++i) {
+            const int32_t v = in[i];
+            if (v > last) a[m++] = v;
+            last = max(last, v);
+        }
+    };
+    constexpr int kLocal = 96;  // lists up to this long are sorted in local memory
+    if (n <= kLocal) {
+        int32_t loc[kLocal];
+        sort(loc, a);
+        pack(loc);
+    } else {
+        sort(a, a);
+        pack(a);
+    }
     S.deg[g] = m;
 }
 
@@ -171,7 +252,65 @@ __global__ void k_smirror(SmoothBatch S) {
     }
 }
 
-/* ---------------- the bound and its adjoint: one CTA per instance ------- */
+/* ---------------- lists by ascending cost -------------------------------- */
+// A node root reads its list in ascending cost and stops early, so each list
+// is stored a second time sorted by (cost, neighbour): sent holds the cost bits
+// and the local neighbour, splace the entry's place in the CSR row.  The
+// persistent kernel, a lane or two to a node, reads the first entries from
+// slices of 32 lanes (ssell: column j of lane l at 32 j + l, S.W columns), a
+// column with unit stride: from the rows its reads touched a sector a lane
+// (132 ms against 55 for the bound and gradient of 1,024 lattice instances).
+// With four lanes or more to a node, the per-step kernels, the rows are sectors.
+__global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= S.n_total) return;
+    const int64_t r0 = S.row[g];
+    const int n = (int)(S.row[g + 1] - r0);
+    auto key_of = [&](int k) { return ((unsigned long long)__float_as_uint(S.c[r0 + k]) << 32) | (unsigned)k; };
+    auto put = [&](int k, unsigned long long key) {
+        const int place = (int)(unsigned)key;
+        S.sent[r0 + k] = make_uint2((unsigned)(key >> 32), (unsigned)S.nbr[r0 + place]);
+        S.splace[r0 + k] = place;
+    };
+    constexpr int kLocal = 64;
+    if (n <= kLocal) {
+        unsigned long long loc[kLocal];
+        for (int k = 0; k < n; ++k) {
+            const unsigned long long x = key_of(k);
+            int j = k;
+            while (j > 0 && loc[j - 1] > x) { loc[j] = loc[j - 1]; --j; }
+            loc[j] = x;
+        }
+        for (int k = 0; k < n; ++k) put(k, loc[k]);
+        return;
+    }
+    // a long list (a hub): rank each entry among the others
+    for (int k = 0; k < n; ++k) {
+        const unsigned long long x = key_of(k);
+        int rank = 0;
+        for (int j = 0; j < n; ++j) rank += key_of(j) < x;
+        put(rank, x);
+    }
+}
+
+template <int G>
+__global__ void __launch_bounds__(128) k_ssell(SmoothBatch S) {
+    const int64_t w = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= S.n_warps) return;
+    const int lane = threadIdx.x & 31;
+    const int b = find_inst(S.sbase, S.n_inst, w);
+    const int64_t g = S.offs[b] + (w - S.sbase[b]) * (32 / G) + lane / G;
+    const bool in = g < S.offs[b + 1];
+    const int64_t r0 = in ? S.row[g] : 0;
+    const int n = in ? (int)(S.row[g + 1] - r0) : 0;
+    uint2* out = S.sell + w * 32 * S.W + lane;
+    for (int j = 0; j < S.W; ++j) {
+        const int k = j * G + lane % G;
+        out[32 * j] = k < n ? S.sent[r0 + k] : make_uint2(0x7f800000u, 0u);
+    }
+}
+
+/* ---------------- node roots over the entries within reach --------------- */
 __device__ __forceinline__ double sigm(double z) {
     if (z >= 0) return 1.0 / (1.0 + exp(-z));
     const double e = exp(z);
@@ -180,8 +319,8 @@ __device__ __forceinline__ double sigm(double z) {
 __device__ __forceinline__ double softplus(double z) { return fmax(z, 0.0) + log1p(exp(-fabs(z))); }
 // sigma(z) (1 - sigma(z)) without cancellation
 __device__ __forceinline__ double dsig(double z) {
-    const double e = exp(-fabs(z));
-    return (e / (1.0 + e)) * (1.0 / (1.0 + e));
+    const double e = exp(-fabs(z)), big = 1.0 / (1.0 + e);
+    return e * big * big;
 }
 
 // sum_k sigma(z_k) - 2 without cancellation: each term splits into its
@@ -192,7 +331,7 @@ struct LogitAcc {
     double cnt = 0, tail = 0, scale = 0, slope = 0;
     __device__ __forceinline__ void add(double z) {
         const double e = exp(-fabs(z));
-        const double m = e / (1.0 + e), big = 1.0 / (1.0 + e);
+        const double big = 1.0 / (1.0 + e), m = e * big;
         if (z >= 0) { cnt += 1.0; tail -= m; } else { tail += m; }
         scale += m;
         slope += m * big;
@@ -216,39 +355,301 @@ __device__ __forceinline__ double root_step(const LogitAcc& r, double tau, doubl
     return sn;
 }
 
-__device__ double node_root(const int32_t* nb, const float* c, int n, const double* u, double tau,
-                            int max_it, unsigned long long& terms) {
-    double m0 = INFINITY, m1 = INFINITY, m2 = INFINITY;
-    for (int k = 0; k < n; ++k) top3_insert((double)c[k] - u[nb[k]], m0, m1, m2);
-    double lo = m0 - 40 * tau, hi = m2 + 40 * tau;
+// Which entries a root needs.  With m2 the third smallest a_k, the root is at
+// most m2 + tau ln 2 (three sigmas of 2/3 there), and a Newton step is at most
+// 2 tau long (a remainder's slope is at least half the remainder), so no point
+// the sums are taken at lies above m2 + 3 tau.  An entry past m2 + kReach tau
+// then adds less than e^-(kReach - 3) of what the third smallest adds to the
+// scale of the residual: 64 of them stay below 3e-19 of it, where FP64 rounds
+// at 1e-16.  They are left out; with tau at a hundredth of the point spacing
+// three to five of some thirty entries remain.  Since a_k >= c_k - max u, the
+// scan of the ascending costs ends at the first c_k above that bound.
+constexpr double kReach = 50.0;
+constexpr int kBuf = 12;  // entries within reach that a lane keeps in shared memory
+
+// A group of G lanes holds a node, lane l its entries l, l + G, ...: the lanes'
+// reads of a column fill sectors, their exponentials run side by side, and sums
+// and selections take log2 G shuffles.  Every lane of a warp takes part in the
+// shuffles; a group without a node has an empty list.
+// One lane's part of a list: get(j) its j-th entry, acc(j) where its share of
+// dL/dc is summed; n entries.
+template <int G>
+struct RowPart {
+    int n, deg;
+    const uint2* ent;
+    double* gs;
+    __device__ __forceinline__ uint2 get(int j) const { return ent[j * G]; }
+    __device__ __forceinline__ double& acc(int j) const { return gs[j * G]; }
+};
+template <int G>
+struct SlicePart {
+    int n, deg, W;
+    const uint2* col;     // the lane's column of its slice
+    double* gcol;
+    RowPart<G> row;       // the entries past W
+    __device__ __forceinline__ uint2 get(int j) const { return j < W ? col[32 * j] : row.get(j); }
+    __device__ __forceinline__ double& acc(int j) const { return j < W ? gcol[32 * j] : row.acc(j); }
+};
+// of node v of the instance that starts at node `base` (no entries: in = false)
+template <int G>
+__device__ __forceinline__ RowPart<G> row_part(const SmoothBatch& S, int64_t base, int v, bool in) {
+    RowPart<G> p{0, 0, nullptr, nullptr};
+    if (in) {
+        const int l = threadIdx.x % G;
+        const int64_t r0 = S.row[base + v];
+        p.deg = (int)(S.row[base + v + 1] - r0);
+        p.n = (p.deg - l + G - 1) / G;
+        p.ent = S.sent + r0 + l;
+        p.gs = S.gs + r0 + l;
+    }
+    return p;
+}
+template <int G>
+__device__ __forceinline__ SlicePart<G> slice_part(const SmoothBatch& S, int64_t base, int64_t w0, int v, bool in) {
+    SlicePart<G> p;
+    p.row = row_part<G>(S, base, v, in);
+    p.n = p.row.n;
+    p.deg = p.row.deg;
+    p.W = S.W;
+    const int64_t at = (w0 + v / (32 / G)) * 32 * S.W + (threadIdx.x & 31);
+    p.col = S.sell + at;
+    p.gcol = S.gsell + at;
+    return p;
+}
+template <int G>
+__device__ __forceinline__ double grp_sum(double x) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+// the three smallest of two sorted triples
+__device__ __forceinline__ void low3_merge(double& m0, double& m1, double& m2, double p0, double p1, double p2) {
+    const double n0 = dmin2(m0, p0);
+    const double n1 = dmin2(dmin2(m1, p1), dmax2(m0, p0));
+    m2 = dmin2(dmin2(m2, p2), dmin2(dmax2(m1, p0), dmax2(m0, p1)));
+    m0 = n0;
+    m1 = n1;
+}
+template <int G>
+__device__ __forceinline__ void grp_low3(double& m0, double& m1, double& m2) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+        low3_merge(m0, m1, m2, __shfl_xor_sync(0xffffffffu, m0, o), __shfl_xor_sync(0xffffffffu, m1, o),
+                   __shfl_xor_sync(0xffffffffu, m2, o));
+}
+
+// Scratch of one lane: up to cap values and their 16-bit indices, strided so
+// that a warp's accesses do not conflict.
+struct SBuf {
+    double* x;
+    uint16_t* i;
+    int stride, cap;
+    __device__ __forceinline__ void push(int& cnt, double v, int k) const {
+        if (cnt < cap) { x[cnt * stride] = v; i[cnt * stride] = (uint16_t)k; }
+        ++cnt;
+    }
+};
+
+// Max of the lanes' x into *slot, as an ordered integer.
+__device__ __forceinline__ long long ord_of(double x) {
+    const long long i = __double_as_longlong(x);
+    return i ^ ((i >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double ord_to(long long i) {
+    return __longlong_as_double(i ^ ((i >> 63) & 0x7fffffffffffffffll));
+}
+constexpr long long kOrdLow = -0x7ff0000000000001ll;  // ord_of(-inf)
+__device__ __forceinline__ void warp_ord_max(double x, long long* slot) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(slot, ord_of(x));
+}
+
+// The root of a node given the potentials u and a bound umax >= every u; *thr
+// receives m2 + kReach tau.  terms counts the list terms the sums cover.
+template <int G, class List, class UP>
+__device__ __forceinline__ double node_root(const SmoothBatch& S, const List& L, UP u, double umax, const SBuf& B,
+                                            double* thr, unsigned long long& terms) {
+    constexpr int C = G >= 8 ? 2 : 4;  // columns read at once
+    const bool lead = threadIdx.x % G == 0;
+    const double win = kReach * S.tau;
+    auto cost = [&](const uint2& e) { return (double)__uint_as_float(e.x); };
+    double m0 = INFINITY, m1 = INFINITY, m2 = INFINITY;  // of this lane's entries so far
+    double bound = INFINITY;                             // at least m2 of the node + win
+    int cnt = 0, end = 0;
+    while (end < L.n) {
+        uint2 e[C];
+        double a[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) e[i] = end + i < L.n ? L.get(end + i) : make_uint2(0x7f800000u, 0u);
+#pragma unroll
+        for (int i = 0; i < C; ++i) a[i] = cost(e[i]) - u[e[i].y];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            top3_insert(a[i], m0, m1, m2);
+            bound = dmin2(bound, m2 + win);
+            if (a[i] <= bound && end + i < L.n) B.push(cnt, a[i], end + i);
+        }
+        end = min(end + C, L.n);
+        if (cost(e[C - 1]) - umax > bound) break;
+    }
+    __syncwarp();
+    if (G > 1) grp_low3<G>(m0, m1, m2);
+    const double t = m2 + win;
+    *thr = t;
+    double lo = m0 - 40 * S.tau, hi = m2 + 40 * S.tau;
     double s = 0.5 * (m1 + m2);
-    for (int it = 0; it < max_it; ++it) {
+    bool go = L.deg > 0;
+    for (int it = 0; it < S.newton_max; ++it) {
         LogitAcc r;
-        for (int k = 0; k < n; ++k) r.add((s - ((double)c[k] - u[nb[k]])) / tau);
-        terms += (unsigned long long)n;
-        const double sn = root_step(r, tau, s, lo, hi);
-        if (sn != sn) break;
-        s = sn;
+        if (go) {
+            if (lead) terms += (unsigned long long)L.deg;
+            if (cnt <= B.cap) {
+                #pragma unroll 2
+                for (int j = 0; j < cnt; ++j) r.add((s - B.x[j * B.stride]) * S.inv_tau);
+            } else {
+                for (int j = 0; j < end; j += 4) {  // four at a time, their loads and sums side by side
+                    double z[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint2 e = j + i < end ? L.get(j + i) : make_uint2(0x7f800000u, 0u);
+                        const double a = cost(e) - u[e.y];
+                        z[i] = a <= t ? (s - a) * S.inv_tau : -INFINITY;  // adds nothing
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) r.add(z[i]);
+                }
+            }
+        }
+        if (G > 1) {
+            __syncwarp();
+            r.cnt = grp_sum<G>(r.cnt);
+            r.tail = grp_sum<G>(r.tail);
+            r.scale = grp_sum<G>(r.scale);
+            r.slope = grp_sum<G>(r.slope);
+        }
+        if (go) {
+            const double sn = root_step(r, S.tau, s, lo, hi);
+            if (sn != sn) go = false;
+            else s = sn;
+        }
+        if (G > 1 ? !__any_sync(0xffffffffu, go) : !go) break;
     }
     return s;
 }
 
-struct SInst {
-    int V;
-    int64_t base;
-    const int64_t* row;  // row + base
-    int64_t r0;
-};
-
-// One damped Jacobi step u -> un; writes the roots to s_out when given.
-__device__ __forceinline__ void sjacobi(const SmoothBatch& S, const SInst& I, const double* u,
-                                        double* un, double* s_out, unsigned long long& terms) {
-    for (int v = threadIdx.x; v < I.V; v += kST) {
-        const int64_t a = I.row[v], e = I.row[v + 1];
-        const double s = node_root(S.nbr + a, S.c + a, (int)(e - a), u, S.tau, S.newton_max, terms);
-        if (s_out) s_out[v] = s;
-        un[v] = (1.0 - S.omega) * u[v] + S.omega * s;
+// Reverse pass 1 of one step: mu_v = omega lam_v / D_v with D_v = sum p_e over
+// the entries within reach (p falls off as the remainders do), and
+// q_e = mu_v p_e added to the node's share of dL/dc.
+template <int G, class List, class UP>
+__device__ __forceinline__ double node_rev1(const SmoothBatch& S, const List& L, UP u, double umax, const SBuf& B,
+                                            double s, double thr, double lam, unsigned long long& terms) {
+    constexpr int C = G >= 8 ? 2 : 4;
+    int cnt = 0, end = 0;
+    while (end < L.n) {
+        uint2 e[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) e[i] = end + i < L.n ? L.get(end + i) : make_uint2(0x7f800000u, 0u);
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const double a = (double)__uint_as_float(e[i].x) - u[e[i].y];
+            if (a <= thr && end + i < L.n) B.push(cnt, a, end + i);
+        }
+        end = min(end + C, L.n);
+        if ((double)__uint_as_float(e[C - 1].x) - umax > thr) break;
     }
+    if (threadIdx.x % G == 0) terms += (unsigned long long)L.deg;
+    double D = 0.0;
+    auto p_of = [&](double a) { return dsig((s - a) * S.inv_tau) * S.inv_tau; };
+    auto each = [&](auto f) {  // entries within reach, re-read
+        for (int j = 0; j < end; ++j) {
+            const uint2 e = L.get(j);
+            const double a = (double)__uint_as_float(e.x) - u[e.y];
+            if (a <= thr) f(j, a);
+        }
+    };
+    if (cnt <= B.cap) {
+        for (int j = 0; j < cnt; ++j) {
+            const double p = p_of(B.x[j * B.stride]);
+            B.x[j * B.stride] = p;
+            D += p;
+        }
+    } else {
+        each([&](int, double a) { D += p_of(a); });
+    }
+    __syncwarp();
+    D = grp_sum<G>(D);
+    const double mu = D > 0 ? S.omega * lam / D : 0.0;  // D == 0: all saturated
+    if (cnt <= B.cap) {
+        for (int j = 0; j < cnt; ++j) L.acc(B.i[j * B.stride]) += mu * B.x[j * B.stride];
+    } else {
+        each([&](int j, double a) { L.acc(j) += mu * p_of(a); });
+    }
+    return mu;
+}
+// Reverse pass 2: what the neighbours v that hold node w within their reach
+// (a = c - u_w at most thr_v) take from lam_w: the sum of mu_v p over them, p
+// formed from the same operands as in pass 1, so q need not be stored.
+template <int G, class List, class TP, class SP, class MP>
+__device__ __forceinline__ double node_rev2(const SmoothBatch& S, const List& L, double uw, double thrmax, TP thr,
+                                            SP s, MP mu, const SBuf& B) {
+    constexpr int C = G >= 8 ? 2 : 4;
+    int cnt = 0, end = 0;
+    while (end < L.n) {
+        uint2 e[C];
+#pragma unroll
+        for (int i = 0; i < C; ++i) e[i] = end + i < L.n ? L.get(end + i) : make_uint2(0x7f800000u, 0u);
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const double a = (double)__uint_as_float(e[i].x) - uw;
+            if (end + i < L.n && a <= thr[e[i].y]) B.push(cnt, a, (int)e[i].y);
+        }
+        end = min(end + C, L.n);
+        if ((double)__uint_as_float(e[C - 1].x) - uw > thrmax) break;
+    }
+    double sum = 0.0;
+    auto q_of = [&](int v, double a) { return mu[v] * (dsig((s[v] - a) * S.inv_tau) * S.inv_tau); };
+    if (cnt <= B.cap) {
+        for (int j = 0; j < cnt; ++j) sum += q_of(B.i[j * B.stride], B.x[j * B.stride]);
+    } else {
+        for (int j = 0; j < end; ++j) {
+            const uint2 e = L.get(j);
+            const double a = (double)__uint_as_float(e.x) - uw;
+            if (a <= thr[e.y]) sum += q_of((int)e.y, a);
+        }
+    }
+    __syncwarp();
+    return grp_sum<G>(sum);
+}
+
+/* ---------------- the bound and its adjoint: one CTA per instance ------- */
+struct SInst {
+    int b, V;
+    int64_t base, w0;    // first node, first slice
+    const int64_t* row;  // row + base
+};
+constexpr int kCG = 1;  // lanes of a node
+
+// One damped Jacobi step u -> un; writes the roots and the reach bounds when
+// given, and the largest new potential into *umax_next.
+__device__ __forceinline__ void sjacobi(const SmoothBatch& S, const SInst& I, const double* u, double* un,
+                                        double* s_out, double* t_out, const SBuf& B, double umax,
+                                        long long* umax_next, unsigned long long& terms) {
+    double mx = -INFINITY;
+    const int v1 = (I.V + 32 / kCG - 1) / (32 / kCG) * (32 / kCG);  // whole warps
+    for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
+        const auto nd = slice_part<kCG>(S, I.base, I.w0, v, v < I.V);
+        double thr;
+        const double s = node_root<kCG>(S, nd, u, umax, B, &thr, terms);
+        if (v < I.V && threadIdx.x % kCG == 0) {
+            if (s_out) { s_out[v] = s; t_out[v] = thr; }
+            const double x = (1.0 - S.omega) * u[v] + S.omega * s;
+            un[v] = x;
+            mx = fmax(mx, x);
+        }
+        __syncwarp();
+    }
+    warp_ord_max(mx, umax_next);
 }
 
 __device__ double sbound(const SmoothBatch& S, const SInst& I, const double* u, double* sred,
@@ -266,51 +667,66 @@ __device__ double sbound(const SmoothBatch& S, const SInst& I, const double* u, 
     return su - S.tau * sp;
 }
 
+// What bounds it: the scans of the list heads (a column read, a gathered
+// potential and the top-3 insertion an entry) and the few exponentials a root
+// needs, and for the last instances of a batch the latency of their 300
+// dependent passes.  Two 512-thread CTAs an SM: 40.9 ms for 1,024 lattice
+// instances of 200-2,000 points (N = 24, tau 1e-3, 100 steps, gradient), 49.7
+// with four of 256 threads, 47.1 with one of 1,024; 347 ms with a thread per
+// node over the whole CSR row, an exponential and two divisions an entry.
 template <bool GRAD>
-__global__ void __launch_bounds__(kST) k_sbound(SmoothBatch S) {
+__global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int max_v) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double sred[kST / 32];
     __shared__ int sitem;
+    __shared__ long long smax[3], stmax[2];  // largest potential (three steps), largest reach bound
     double* Ha = reinterpret_cast<double*>(smem_raw);
-    // logistic terms this thread evaluated (exp-based: Newton sums, softplus,
-    // sigma, sigma'), added to S.work when the queue is empty
+    double* bx = Ha + 2 * (size_t)max_v;
+    const SBuf B{bx + threadIdx.x, reinterpret_cast<uint16_t*>(bx + (size_t)cap * kST) + threadIdx.x, kST, cap};
+    // list terms the sums of this thread cover (Newton sums, softplus, sigma,
+    // sigma'), added to S.work when the queue is empty
     unsigned long long terms = 0;
     for (;;) {
         if (threadIdx.x == 0) sitem = atomicAdd(S.queue, 1);
         __syncthreads();
-        const int b = sitem;
+        const int item = sitem;
         __syncthreads();
-        if (b >= S.n_inst) {
+        if (item >= S.n_inst) {
             if (S.work && terms) atomicAdd(S.work, terms);
             return;
         }
         SInst I;
-        I.base = S.offs[b];
-        I.V = (int)(S.offs[b + 1] - I.base);
+        I.b = S.order[item];
+        I.base = S.offs[I.b];
+        I.V = (int)(S.offs[I.b + 1] - I.base);
         I.row = S.row + I.base;
-        I.r0 = I.row[0];
-        double* Hb = Ha + I.V;
+        I.w0 = S.sbase[I.b];
+        const int v1 = (I.V + 32 / kCG - 1) / (32 / kCG) * (32 / kCG);
+        double* Hb = Ha + max_v;
         const int T = S.iters, K = S.ckpt;
         double* ck = S.ck + I.base * S.n_ck;
         for (int v = threadIdx.x; v < I.V; v += kST) Ha[v] = 0.0;
+        if (threadIdx.x == 0) { smax[0] = ord_of(0.0); smax[1] = smax[2] = kOrdLow; }
         __syncthreads();
         double* u = Ha;
         double* un = Hb;
         for (int t = 0; t < T; ++t) {
             if (GRAD && t % K == 0)
                 for (int v = threadIdx.x; v < I.V; v += kST) ck[(t / K) * I.V + v] = u[v];
-            sjacobi(S, I, u, un, nullptr, terms);
+            if (threadIdx.x == 0) smax[(t + 2) % 3] = kOrdLow;
+            sjacobi(S, I, u, un, nullptr, nullptr, B, ord_to(smax[t % 3]), &smax[(t + 1) % 3], terms);
             __syncthreads();
             double* tt = u; u = un; un = tt;
         }
         const double L = sbound(S, I, u, sred, terms);
-        if (threadIdx.x == 0) S.L[b] = L;
+        if (threadIdx.x == 0) S.L[I.b] = L;
         if (!GRAD) { __syncthreads(); continue; }
         // adjoint of L(u^T) with respect to u^T and (explicitly) c; the
         // explicit sigma_e is split evenly over the edge's two slots
-        const double up = S.dL[b];
+        const double up = S.dL[I.b];
         double* lam = S.lam + I.base;
         double* lam2 = S.lam2 + I.base;
+        double* mu = S.mu + I.base;
         for (int v = threadIdx.x; v < I.V; v += kST) {
             LogitAcc r;
             for (int64_t k = I.row[v]; k < I.row[v + 1]; ++k) {
@@ -324,83 +740,162 @@ __global__ void __launch_bounds__(kST) k_sbound(SmoothBatch S) {
         __syncthreads();
         double* su_ = S.segu + I.base * K;
         double* ss_ = S.segs + I.base * K;
+        double* st_ = S.segt + I.base * K;
+        double* sm_ = S.segm + (int64_t)I.b * K;  // largest potential of each stored iterate
         const int nseg = (T + K - 1) / K;
         for (int seg = nseg - 1; seg >= 0; --seg) {
             const int t0 = seg * K, t1 = min(T, t0 + K);
-            for (int v = threadIdx.x; v < I.V; v += kST) Ha[v] = ck[seg * I.V + v];
+            if (threadIdx.x == 0) smax[0] = smax[1] = smax[2] = kOrdLow;
+            __syncthreads();
+            double mx = -INFINITY;
+            for (int v = threadIdx.x; v < I.V; v += kST) {
+                const double x = ck[seg * I.V + v];
+                Ha[v] = x;
+                mx = fmax(mx, x);
+            }
+            warp_ord_max(mx, &smax[0]);
             __syncthreads();
             u = Ha;
             un = Hb;
             for (int t = t0; t < t1; ++t) {  // recompute the segment's iterates
-                double* ut = su_ + (t - t0) * I.V;
+                const int j = t - t0;
+                double* ut = su_ + (int64_t)j * I.V;
                 for (int v = threadIdx.x; v < I.V; v += kST) ut[v] = u[v];
-                sjacobi(S, I, u, un, ss_ + (t - t0) * I.V, terms);
+                if (threadIdx.x == 0) { smax[(j + 2) % 3] = kOrdLow; sm_[j] = ord_to(smax[j % 3]); }
+                sjacobi(S, I, u, un, ss_ + (int64_t)j * I.V, st_ + (int64_t)j * I.V, B, ord_to(smax[j % 3]),
+                        &smax[(j + 1) % 3], terms);
                 __syncthreads();
                 double* tt = u; u = un; un = tt;
             }
             for (int t = t1 - 1; t >= t0; --t) {
-                const double* ut = su_ + (t - t0) * I.V;
-                const double* st = ss_ + (t - t0) * I.V;
-                // pass 1: mu_v = omega lam_v / D_v; q = mu_v p_e on v's slots
+                const int j = t - t0;
+                const double* ut = su_ + (int64_t)j * I.V;
+                const double* st = ss_ + (int64_t)j * I.V;
+                const double* tv = st_ + (int64_t)j * I.V;
+                if (threadIdx.x == 0) stmax[t & 1] = kOrdLow;
+                __syncthreads();
+                // the iterate and its reach bounds in shared memory
+                double tm = -INFINITY;
                 for (int v = threadIdx.x; v < I.V; v += kST) {
-                    const int64_t a = I.row[v], e = I.row[v + 1];
-                    double D = 0.0;
-                    for (int64_t k = a; k < e; ++k) {
-                        const double p = dsig((st[v] + ut[S.nbr[k]] - (double)S.c[k]) / S.tau) / S.tau;
-                        S.q[k] = p;
-                        D += p;
-                    }
-                    terms += (unsigned long long)(e - a);
-                    const double mu = D > 0 ? S.omega * lam[v] / D : 0.0;  // D == 0: all saturated
-                    for (int64_t k = a; k < e; ++k) {
-                        const double qk = mu * S.q[k];
-                        S.q[k] = qk;
-                        S.gc[k] += qk;
-                    }
+                    Ha[v] = ut[v];
+                    const double x = tv[v];
+                    Hb[v] = x;
+                    tm = fmax(tm, x);
+                }
+                warp_ord_max(tm, &stmax[t & 1]);
+                __syncthreads();
+                const double umax = sm_[j], thrmax = ord_to(stmax[t & 1]);
+                const bool lead = threadIdx.x % kCG == 0;
+                for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
+                    const bool in = v < I.V;
+                    const auto nd = slice_part<kCG>(S, I.base, I.w0, v, in);
+                    const double m = node_rev1<kCG>(S, nd, (const double*)Ha, umax, B, in ? st[v] : 0.0,
+                                                    in ? Hb[v] : 0.0, in ? lam[v] : 0.0, terms);
+                    if (in && lead) mu[v] = m;
+                    __syncwarp();
                 }
                 __syncthreads();
-                // pass 2: lam_w <- (1 - omega) lam_w - sum over w's edges of the
-                // neighbour's q on the same edge
-                for (int w = threadIdx.x; w < I.V; w += kST) {
-                    double l = (1.0 - S.omega) * lam[w];
-                    for (int64_t k = I.row[w]; k < I.row[w + 1]; ++k) l -= S.q[S.mirror[k]];
-                    lam2[w] = l;
+                for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
+                    const bool in = v < I.V;
+                    const auto nd = slice_part<kCG>(S, I.base, I.w0, v, in);
+                    const double x = node_rev2<kCG>(S, nd, in ? Ha[v] : 0.0, thrmax, (const double*)Hb, st,
+                                                    (const double*)mu, B);
+                    if (in && lead) lam2[v] = (1.0 - S.omega) * lam[v] - x;
+                    __syncwarp();
                 }
                 __syncthreads();
                 double* tt = lam; lam = lam2; lam2 = tt;
             }
         }
-        // dL/dc_e = both slots' sums; chain through c_e = |p_v - p_w|
-        for (int v = threadIdx.x; v < I.V; v += kST) {
-            const int64_t gv = I.base + v;
-            const double xv = S.x[gv], yv = S.y[gv];
-            double gx = 0.0, gy = 0.0;
-            for (int64_t k = I.row[v]; k < I.row[v + 1]; ++k) {
-                const double ce = (double)S.c[k];
-                if (ce == 0.0) continue;
-                const int64_t gw = I.base + S.nbr[k];
-                const double dc = S.gc[k] + S.gc[S.mirror[k]];
-                gx += dc * (xv - (double)S.x[gw]) / ce;
-                gy += dc * (yv - (double)S.y[gw]) / ce;
-            }
-            S.gx[gv] = (float)gx;
-            S.gy[gv] = (float)gy;
-        }
-        __syncthreads();
     }
 }
 
-/* ---------------- one launch per step: a warp per node, all instances ---- */
-// The root of a node with a warp: lanes hold four a_k each in registers (the
-// first 128 list entries; later ones are re-read), top-3 and the Newton sums
-// by XOR butterflies, which give every lane the same bits, so the whole warp
-// follows one Newton path.
+/* ---------------- one launch per step, all instances --------------------- */
+// G lanes per node, each instance's nodes from a whole warp on (sbase counts
+// warps); the potentials stay in global memory.  Few nodes leave SMs idle, so
+// more lanes share a node's exponentials; many nodes fill them, and the shuffles
+// of a wide group are wasted.  Bound and gradient (100 steps, N = 24) at G = 4 /
+// 8 / 16 / 32: 500 points 4.4 / 3.4 / 2.8 / 2.6 ms, 4,000 points 5.5 / 4.1 / 3.6
+// / 3.8, 10,000 points 6.0 / 5.5 / 5.9 / 7.0, 64 instances of 70,000 points in
+// all 8.7 / 10.9 / 16.0 / 22.0.
+constexpr int kWT = 128;  // threads of a CTA
+static int steps_lanes(int64_t n_total) {
+    return n_total <= 3000 ? 32 : (n_total <= 7000 ? 16 : (n_total <= 14000 ? 8 : 4));
+}
+template <int kWG>
+struct SThread {
+    RowPart<kWG> nd;
+    int b;
+    int64_t g, base;
+    bool in, lead;
+};
+template <int kWG>
+__device__ __forceinline__ bool step_thread(const SmoothBatch& S, SThread<kWG>& t) {
+    const int64_t w = (int64_t)blockIdx.x * (kWT / 32) + (threadIdx.x >> 5);
+    if (w >= S.n_warps) return false;
+    t.b = find_inst(S.sbase, S.n_inst, w);
+    t.base = S.offs[t.b];
+    const int v = (int)(w - S.sbase[t.b]) * (32 / kWG) + (threadIdx.x & 31) / kWG;
+    t.g = t.base + v;
+    t.in = t.g < S.offs[t.b + 1];
+    t.lead = t.in && threadIdx.x % kWG == 0;
+    t.nd = row_part<kWG>(S, t.base, v, t.in);
+    return true;
+}
+#define F2M_SBUF                                                         \
+    __shared__ double s_bx[kBuf * kWT];                                  \
+    __shared__ uint16_t s_bi[kBuf * kWT];                                \
+    const SBuf B{s_bx + threadIdx.x, s_bi + threadIdx.x, kWT, kBuf}
+
+// u -> un for every node; stores u (ust), the roots (sst) and the reach bounds
+// (tst) when given, and checkpoints u at index ck (>= 0).  umax / umax_next:
+// the largest potential of each instance, before and after.
+template <int kWG>
+__global__ void __launch_bounds__(kWT) k_sw_step(SmoothBatch S, const double* u, double* un, double* ust, double* sst,
+                                                 double* tst, int ck, const long long* umax, long long* umax_next) {
+    F2M_SBUF;
+    SThread<kWG> t;
+    if (!step_thread(S, t)) return;
+    double mx = -INFINITY, thr;
+    unsigned long long terms = 0;
+    const double s = node_root<kWG>(S, t.nd, u + t.base, ord_to(umax[t.b]), B, &thr, terms);
+    if (t.lead) {
+        const int64_t g = t.g;
+        const double uv = u[g];
+        if (ck >= 0) S.ck[(int64_t)ck * S.n_total + g] = uv;
+        if (ust) ust[g] = uv;
+        if (sst) { sst[g] = s; tst[g] = thr; }
+        mx = (1.0 - S.omega) * uv + S.omega * s;
+        un[g] = mx;
+    }
+    __syncwarp();
+    warp_ord_max(mx, umax_next + t.b);
+}
+
+// u = 0 (ck < 0) or a checkpoint, and its largest value per instance
+template <int kWG>
+__global__ void __launch_bounds__(kWT) k_sw_init(SmoothBatch S, double* u, int ck, long long* umax) {
+    SThread<kWG> t;
+    if (!step_thread(S, t)) return;
+    double x = -INFINITY;
+    if (t.lead) {
+        x = ck < 0 ? 0.0 : S.ck[(int64_t)ck * S.n_total + t.g];
+        u[t.g] = x;
+    }
+    __syncwarp();
+    warp_ord_max(x, umax + t.b);
+}
+// the per-instance maxima of every step, reset
+__global__ void k_sw_low(long long* m, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) m[i] = kOrdLow;
+}
+
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     return x;
 }
-
 struct WNode {
     int64_t g, base, r0;
     int n;
@@ -413,73 +908,6 @@ __device__ __forceinline__ bool warp_node(const SmoothBatch& S, WNode& W) {
     W.r0 = S.row[W.g];
     W.n = (int)(S.row[W.g + 1] - W.r0);
     return true;
-}
-
-__device__ double warp_root(const SmoothBatch& S, const WNode& W, const double* u) {
-    const int lane = threadIdx.x & 31;
-    double a[4];
-    double m0 = INFINITY, m1 = INFINITY, m2 = INFINITY;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = lane + 32 * j;
-        a[j] = INFINITY;
-        if (k < W.n) {
-            a[j] = (double)S.c[W.r0 + k] - u[W.base + S.nbr[W.r0 + k]];
-            top3_insert(a[j], m0, m1, m2);
-        }
-    }
-    for (int k = lane + 128; k < W.n; k += 32)
-        top3_insert((double)S.c[W.r0 + k] - u[W.base + S.nbr[W.r0 + k]], m0, m1, m2);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double p0 = __shfl_xor_sync(0xffffffffu, m0, o);
-        const double p1 = __shfl_xor_sync(0xffffffffu, m1, o);
-        const double p2 = __shfl_xor_sync(0xffffffffu, m2, o);
-        top3_insert(p0, m0, m1, m2);
-        top3_insert(p1, m0, m1, m2);
-        top3_insert(p2, m0, m1, m2);
-    }
-    double lo = m0 - 40 * S.tau, hi = m2 + 40 * S.tau;
-    double s = 0.5 * (m1 + m2);
-    for (int it = 0; it < S.newton_max; ++it) {
-        LogitAcc r;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (lane + 32 * j < W.n) r.add((s - a[j]) / S.tau);
-        for (int k = lane + 128; k < W.n; k += 32)
-            r.add((s - ((double)S.c[W.r0 + k] - u[W.base + S.nbr[W.r0 + k]])) / S.tau);
-        r.cnt = warp_sum(r.cnt);
-        r.tail = warp_sum(r.tail);
-        r.scale = warp_sum(r.scale);
-        r.slope = warp_sum(r.slope);
-        const double sn = root_step(r, S.tau, s, lo, hi);
-        if (sn != sn) break;
-        s = sn;
-    }
-    return s;
-}
-
-// u -> un for every node; stores u (ust) and the roots (sst) when given, and
-// checkpoints u and the previous roots at index ck (>= 0).
-__global__ void __launch_bounds__(256) k_sw_step(SmoothBatch S, const double* u, double* un,
-                                                 double* ust, double* sst, int ck) {
-    WNode W;
-    if (!warp_node(S, W)) return;
-    if ((threadIdx.x & 31) == 0) {
-        if (ck >= 0) S.ck[(int64_t)ck * S.n_total + W.g] = u[W.g];
-        if (ust) ust[W.g] = u[W.g];
-    }
-    const double s = warp_root(S, W, u);
-    if ((threadIdx.x & 31) == 0) {
-        if (sst) sst[W.g] = s;
-        un[W.g] = (1.0 - S.omega) * u[W.g] + S.omega * s;
-    }
-}
-
-__global__ void k_sw_init(SmoothBatch S, double* u, int ck) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= S.n_total) return;
-    u[g] = ck < 0 ? 0.0 : S.ck[(int64_t)ck * S.n_total + g];
 }
 
 // per-node terms of L(u^T) and, for the adjoint, lambda^T and the explicit
@@ -523,52 +951,45 @@ __global__ void __launch_bounds__(256) k_sw_sumL(SmoothBatch S) {
     if (threadIdx.x == 0) S.L[b] = x;
 }
 
-__global__ void __launch_bounds__(256) k_sw_rev1(SmoothBatch S, const double* ut, const double* st,
-                                                 const double* lam) {
-    WNode W;
-    if (!warp_node(S, W)) return;
-    const int lane = threadIdx.x & 31;
-    double p[4];
-    double D = 0.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = lane + 32 * j;
-        p[j] = 0.0;
-        if (k < W.n) {
-            p[j] = dsig((st[W.g] + ut[W.base + S.nbr[W.r0 + k]] - (double)S.c[W.r0 + k]) / S.tau) / S.tau;
-            D += p[j];
-        }
-    }
-    auto pk = [&](int k) {
-        return dsig((st[W.g] + ut[W.base + S.nbr[W.r0 + k]] - (double)S.c[W.r0 + k]) / S.tau) / S.tau;
-    };
-    for (int k = lane + 128; k < W.n; k += 32) D += pk(k);
-    D = warp_sum(D);
-    const double mu = D > 0 ? S.omega * lam[W.g] / D : 0.0;  // D == 0: every sigma saturated
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = lane + 32 * j;
-        if (k < W.n) {
-            const double q = mu * p[j];
-            S.q[W.r0 + k] = q;
-            S.gc[W.r0 + k] += q;
-        }
-    }
-    for (int k = lane + 128; k < W.n; k += 32) {
-        const double q = mu * pk(k);
-        S.q[W.r0 + k] = q;
-        S.gc[W.r0 + k] += q;
-    }
+template <int kWG>
+__global__ void __launch_bounds__(kWT) k_sw_rev1(SmoothBatch S, const double* ut, const double* st, const double* tv,
+                                                 const double* lam, const long long* umax, long long* thrmax) {
+    F2M_SBUF;
+    SThread<kWG> t;
+    if (!step_thread(S, t)) return;
+    unsigned long long terms = 0;
+    const double thr = t.in ? tv[t.g] : -INFINITY;
+    const double mu = node_rev1<kWG>(S, t.nd, ut + t.base, ord_to(umax[t.b]), B, t.in ? st[t.g] : 0.0, thr,
+                                     t.in ? lam[t.g] : 0.0, terms);
+    if (t.lead) S.mu[t.g] = mu;
+    __syncwarp();
+    warp_ord_max(thr, thrmax + t.b);
 }
 
-__global__ void __launch_bounds__(256) k_sw_rev2(SmoothBatch S, const double* lam, double* lam2) {
-    WNode W;
-    if (!warp_node(S, W)) return;
-    const int lane = threadIdx.x & 31;
-    double x = 0.0;
-    for (int k = lane; k < W.n; k += 32) x += S.q[S.mirror[W.r0 + k]];
-    x = warp_sum(x);
-    if (lane == 0) lam2[W.g] = (1.0 - S.omega) * lam[W.g] - x;
+template <int kWG>
+__global__ void __launch_bounds__(kWT) k_sw_rev2(SmoothBatch S, const double* ut, const double* st, const double* tv,
+                                                 const double* lam, double* lam2, const long long* thrmax) {
+    F2M_SBUF;
+    SThread<kWG> t;
+    if (!step_thread(S, t)) return;
+    const double x = node_rev2<kWG>(S, t.nd, t.in ? ut[t.g] : 0.0, ord_to(thrmax[t.b]), tv + t.base, st + t.base,
+                                    (const double*)S.mu + t.base, B);
+    if (t.lead) lam2[t.g] = (1.0 - S.omega) * lam[t.g] - x;
+}
+
+// the steps' shares of dL/dc added to the slots
+__global__ void __launch_bounds__(128) k_s_merge(SmoothBatch S) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= S.n_total) return;
+    const int64_t r0 = S.row[g], r1 = S.row[g + 1];
+    int64_t at = 0;
+    if (S.W) {
+        const int b = find_inst(S.offs, S.n_inst, g);
+        const int v = (int)(g - S.offs[b]);
+        at = (S.sbase[b] + v / (32 / kCG)) * 32 * S.W + (v % (32 / kCG)) * kCG;
+    }
+    for (int k = 0; k < (int)(r1 - r0); ++k)
+        S.gc[r0 + S.splace[r0 + k]] += k / kCG < S.W ? S.gsell[at + 32 * (k / kCG) + k % kCG] : S.gs[r0 + k];
 }
 
 __global__ void k_sw_coord(SmoothBatch S) {
@@ -609,20 +1030,47 @@ cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStrea
     if ((e = launch_scan(S.deg, S.row, S.n_total, scan_scratch, s, launches)) != cudaSuccess) return e;
     k_scopy<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
     k_smirror<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    k_ssorted<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    *launches += 3;
+    if (S.W) {
+        k_ssell<kCG><<<nblk(S.n_warps, 4), 128, 0, s>>>(S);
+        ++*launches;
+    }
+    return cudaGetLastError();
+}
+// Zeroes the sums of the reverse steps.
+static cudaError_t clear_smooth_sums(const SmoothBatch& S, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(S.gs, 0, sizeof(double) * S.s_cap, s);
+    if (e == cudaSuccess && S.W) e = cudaMemsetAsync(S.gsell, 0, sizeof(double) * S.n_warps * 32 * S.W, s);
+    return e;
+}
+// nodes of a warp of the persistent kernel's slices, or of the per-step kernels
+int smooth_nodes_per_warp(bool steps, int64_t n_total) { return 32 / (steps ? steps_lanes(n_total) : kCG); }
+// dL/dc of every slot, then the coordinates
+static cudaError_t launch_smooth_coord(const SmoothBatch& S, cudaStream_t s, int64_t* launches) {
+    k_s_merge<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    k_sw_coord<<<nblk(S.n_total, 256), 256, 0, s>>>(S);
     *launches += 2;
     return cudaGetLastError();
 }
 
-cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches) {
+template <int G>
+static cudaError_t launch_steps_of(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches) {
     const int64_t n = S.n_total;
-    const unsigned gw = nblk(n, 8), gt = nblk(n, 256);
+    const unsigned gw = nblk(n, 8), gs = nblk(S.n_warps, kWT / 32);
     const int T = S.iters, K = S.ckpt;
     double* u = S.ua;
     double* un = S.ub;
-    k_sw_init<<<gt, 256, 0, s>>>(S, u, -1);
-    ++*launches;
+    // the largest potentials of each instance: iterate t of the forward pass at
+    // t, of a segment's recomputation at T + 1 + t, then the reach bounds
+    auto um = [&](int64_t t) { return S.umax + t * S.n_inst; };
+    const int64_t rows = (grad ? 3 : 1) * (int64_t)(T + 1) + 1;
+    k_sw_low<<<nblk(rows * S.n_inst, 256), 256, 0, s>>>(S.umax, rows * S.n_inst);
+    k_sw_init<G><<<gs, kWT, 0, s>>>(S, u, -1, um(0));
+    *launches += 2;
     for (int t = 0; t < T; ++t) {
-        k_sw_step<<<gw, 256, 0, s>>>(S, u, un, nullptr, nullptr, (grad && t % K == 0) ? t / K : -1);
+        k_sw_step<G><<<gs, kWT, 0, s>>>(S, u, un, nullptr, nullptr, nullptr, (grad && t % K == 0) ? t / K : -1, um(t),
+                                     um(t + 1));
         double* tt = u; u = un; un = tt;
     }
     if (grad) k_sw_final<true><<<gw, 256, 0, s>>>(S, u);
@@ -630,28 +1078,42 @@ cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64
     k_sw_sumL<<<S.n_inst, 256, 0, s>>>(S);
     *launches += T + 2;
     if (!grad) return cudaGetLastError();
+    cudaError_t e = clear_smooth_sums(S, s);
+    if (e != cudaSuccess) return e;
     double* lam = S.lam;
     double* lam2 = S.lam2;
     for (int seg = (T + K - 1) / K - 1; seg >= 0; --seg) {
         const int t0 = seg * K, t1 = min(T, t0 + K);
         u = S.ua;
         un = S.ub;
-        k_sw_init<<<gt, 256, 0, s>>>(S, u, seg);
+        k_sw_init<G><<<gs, kWT, 0, s>>>(S, u, seg, um(T + 1 + t0));
         for (int t = t0; t < t1; ++t) {
-            k_sw_step<<<gw, 256, 0, s>>>(S, u, un, S.segu + (int64_t)(t - t0) * n,
-                                         S.segs + (int64_t)(t - t0) * n, -1);
+            // (the last step of a segment has no reader; its maximum goes to the spare row)
+            k_sw_step<G><<<gs, kWT, 0, s>>>(S, u, un, S.segu + (int64_t)(t - t0) * n, S.segs + (int64_t)(t - t0) * n,
+                                         S.segt + (int64_t)(t - t0) * n, -1, um(T + 1 + t),
+                                         t + 1 < t1 ? um(T + 2 + t) : um(3 * (int64_t)(T + 1)));
             double* tt = u; u = un; un = tt;
         }
         for (int t = t1 - 1; t >= t0; --t) {
-            k_sw_rev1<<<gw, 256, 0, s>>>(S, S.segu + (int64_t)(t - t0) * n, S.segs + (int64_t)(t - t0) * n, lam);
-            k_sw_rev2<<<gw, 256, 0, s>>>(S, lam, lam2);
+            const double* ut = S.segu + (int64_t)(t - t0) * n;
+            const double* st = S.segs + (int64_t)(t - t0) * n;
+            const double* tv = S.segt + (int64_t)(t - t0) * n;
+            k_sw_rev1<G><<<gs, kWT, 0, s>>>(S, ut, st, tv, lam, um(T + 1 + t), um(2 * (int64_t)(T + 1) + t));
+            k_sw_rev2<G><<<gs, kWT, 0, s>>>(S, ut, st, tv, lam, lam2, um(2 * (int64_t)(T + 1) + t));
             double* tt = lam; lam = lam2; lam2 = tt;
         }
         *launches += 1 + 3 * (t1 - t0);
     }
-    k_sw_coord<<<gt, 256, 0, s>>>(S);
-    ++*launches;
-    return cudaGetLastError();
+    return launch_smooth_coord(S, s, launches);
+}
+
+cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches) {
+    switch (steps_lanes(S.n_total)) {
+        case 4: return launch_steps_of<4>(S, grad, s, launches);
+        case 8: return launch_steps_of<8>(S, grad, s, launches);
+        case 16: return launch_steps_of<16>(S, grad, s, launches);
+        default: return launch_steps_of<32>(S, grad, s, launches);
+    }
 }
 
 int32_t smooth_max_nodes() {
@@ -694,23 +1156,30 @@ cudaError_t launch_logit_probe(int blocks, int iters, double* out, cudaStream_t 
 
 cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaStream_t s,
                                 int64_t* launches) {
-    const size_t dyn = (size_t)max_v * 16;
+    int dev = 0, sms = 0, per_sm = 0, lim = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    // two potential arrays, and a thread's scratch where it fits (an instance
+    // near the limit re-reads its lists instead)
+    const size_t pot = (size_t)max_v * 16;
+    const int cap = (int)std::min<size_t>(kBuf, ((size_t)lim - 1024 - pot) / (kST * 10));
+    const size_t dyn = pot + (size_t)cap * kST * 10;
     const void* fn = grad ? (const void*)k_sbound<true> : (const void*)k_sbound<false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kST, dyn);
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     int grid = sms * per_sm;
     if (grid > S.n_inst) grid = S.n_inst;
     if ((e = cudaMemsetAsync(S.queue, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
     if (S.work && (e = cudaMemsetAsync(S.work, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
-    if (grad) k_sbound<true><<<grid, kST, dyn, s>>>(S);
-    else k_sbound<false><<<grid, kST, dyn, s>>>(S);
+    if (grad && (e = clear_smooth_sums(S, s)) != cudaSuccess) return e;
+    if (grad) k_sbound<true><<<grid, kST, dyn, s>>>(S, cap, max_v);
+    else k_sbound<false><<<grid, kST, dyn, s>>>(S, cap, max_v);
     ++*launches;
-    return cudaGetLastError();
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return grad ? launch_smooth_coord(S, s, launches) : cudaSuccess;
 }
 
 }  // namespace f2m
