@@ -814,10 +814,19 @@ void carve_edge_sort(Arena& A, EdgeSort& E, int64_t S) {
     E.xout = A.take<double>((S * 20 + 7) / 8);  // E = S/2 edges x 40 bytes
 }
 
+// A single instance above this many points runs on the whole GPU although one
+// SM could hold it: its 148 CTAs exchange potentials every few steps, but share
+// the work of a step.  Solve phase on one SM / on all: 1,000 points 1.7 / 2.8
+// ms, 2,000 points 4.8 / 4.6, 3,000 points 14.0 / 11.3, 5,000 points 20.8 / 6.3,
+// 8,000 points 33.3 / 7.0.  Without coordinates (f2m_solve_graph) the CTAs' halos
+// are not local, so those keep the one SM.
+constexpr int32_t kGridSingle = 2500;
+
 f2m_status setup_call(f2m_ctx* ctx, DevCall& C, int32_t n_inst, const int64_t* h_offs, int32_t top_k,
-                      const f2m_params& prm, bool own_inputs) {
+                      const f2m_params& prm, bool own_inputs, bool spatial = true) {
     make_plan(C.pl, n_inst, h_offs, top_k);
-    C.grid = C.pl.max_n > solve_max_nodes() || (prm.solver == 2 && n_inst == 1);
+    C.grid = C.pl.max_n > solve_max_nodes() ||
+             (n_inst == 1 && (prm.solver == 2 || (prm.solver == 0 && spatial && C.pl.max_n > kGridSingle)));
     if (C.grid && n_inst > 1)
         return fail(ctx, F2M_ERR_CAPACITY, "batched instances are limited to " +
                                                std::to_string(solve_max_nodes()) +
@@ -1822,7 +1831,7 @@ f2m_status f2m_solve_graph(f2m_ctx* ctx, int32_t n_nodes, int32_t n_edges, const
     const int64_t offs[2] = {0, n_nodes};
     const int32_t cap_n = (int32_t)std::min<int64_t>(256, std::max<int64_t>(3, (S + n_nodes - 1) / n_nodes + 1));
     DevCall C;
-    f2m_status st = setup_call(ctx, C, 1, offs, cap_n, prm, true);
+    f2m_status st = setup_call(ctx, C, 1, offs, cap_n, prm, true, false);
     if (st) return st;
     if (C.B.S_cap < S) return fail(ctx, F2M_ERR_CAPACITY, "graph too dense for the solver's list arrays");
     C.spatial = false;  // no coordinates: the grid solver keeps the caller's node order

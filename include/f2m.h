@@ -57,7 +57,10 @@ typedef struct f2m_params {
     double shift_max;      /* 32 */
     int64_t max_iters;     /* safety cap on Jacobi iterations per solve (not in the reference) */
     int32_t cost_mode;     /* f2m_cost_mode */
-    int32_t solver;        /* 0 auto: a team per instance, the whole GPU above 10,000 points;
+    int32_t solver;        /* 0 auto: a team per instance; a single instance above 2,500 points
+                              (10,000 from f2m_solve_graph) takes the whole GPU;
+                              1: a team up to 10,000 points (one SM: for callers that run many
+                              single solves side by side, on a context per thread);
                               2: the whole-GPU solver for a single instance of any size */
     int64_t grid_spin_limit; /* the whole-GPU solver's grid barrier is a bounded wait: after
                               this many polls a CTA gives up, every CTA leaves the solve and

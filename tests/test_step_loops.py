@@ -47,3 +47,17 @@ def test_costs_outside_the_short_forms_range(ctx, oracle, scale):
     r = ctx.solve_graph(g.n_nodes, g.v1, g.v2, g.D * scale, g.Do, labels=g.label)
     assert r.status == o.status
     assert np.array_equal(r.F, o.F)
+
+
+@pytest.mark.parametrize("solver", [0, 1])
+@pytest.mark.parametrize("n", [2500, 2501, 4097, 8161, 8200, 9999])
+def test_potentials_on_one_sm_and_on_all(ctx, oracle, n, solver):
+    """A single instance moves to the whole GPU above 2,500 points; solver = 1
+    keeps it on one SM."""
+    x, y = synth.uniform_int_points(n, 700 + n)
+    o = oracle.solve_points(x, y, 10, threads=8)
+    r = ctx.solve_points(x, y, 10, params=f2m_b200.default_params(solver=solver))
+    assert r.status == o.status
+    assert np.array_equal(r.F, o.F)
+    lp, st = ctx.solve_batch(np.array([0, n]), x, y, 10, params=f2m_b200.default_params(solver=solver))
+    assert st[0] == o.status and abs(lp[0] - o.lp) <= 1e-12 * o.lp
