@@ -1080,6 +1080,10 @@ __global__ void __launch_bounds__(kGT, 1) k_solve_grid(Batch B, DevParams P, Gri
     __shared__ int snb[kGridMaxCtas];
     __shared__ int snbn[1];
     __shared__ unsigned swm[kGridNbWords];
+    // an invalid instance has no graph; every CTA reads the status before the
+    // first barrier, and it is written after the last
+    const int st = B.status[b];
+    if (st != F2M_OK && !(refit && st == kNeedsHost)) return;
     const Inst I = make_inst(B, b);
     const int V = I.V;
     const int o0 = (int)(((long long)V * blockIdx.x) / gridDim.x);
