@@ -1,7 +1,8 @@
 // f2m_b200 CUDA kernels for sm_100a.
 //
 // Pipeline of one batched call (one CTA = one instance unless noted):
-//   k_prep      1e-3 rounding, de-duplication, compaction, bbox   (FXY.hpp:231-309)
+//   k_round, k_dup, k_prep   1e-3 rounding, de-duplication, compaction, bbox
+//                                                                  (FXY.hpp:231-309)
 //   k_grid_*    per-instance cell grid (counting sort of the points)
 //   k_cutoff    per-node ring cut-off radius (stat pass)          (FXY.hpp:441-534)
 //   k_select    per-node first-N neighbours by (d, emitter, partner)
@@ -30,7 +31,6 @@
 namespace f2m {
 
 constexpr int kT = 256;       // width of the node-parallel kernels
-constexpr int kTile = 1024;   // points per shared-memory tile (16 KB)
 constexpr int kMaxPasses = 64;
 
 __device__ __forceinline__ double round3(double x) {
@@ -39,49 +39,102 @@ __device__ __forceinline__ double round3(double x) {
 }
 
 /* ------------------------------------------------------------------ */
-/* k_prep: rounding, de-duplication, compaction, bbox (FXY.hpp:231-309)  */
+/* k_round, k_dup: rounding and de-duplication (FXY.hpp:252-267)         */
+/* ------------------------------------------------------------------ */
+// A point is dropped if an earlier point has identical rounded coordinates; it
+// maps to the first such point (FXY.hpp:260-265).  An open-addressing table of
+// two places a point (in top_nbr, free until the kNN) holds point indices; equal
+// points meet in one place, which keeps the smallest index, and a second kernel
+// reads it back.  +0 and -0 are equal, NaN equals nothing, as in the
+// comparison.  (Thread per point over the whole GPU: 5,000 points took 2.65 ms
+// as a quadratic pass of one CTA, 100,000 took 4.5 ms as a sort on the host.)
+struct DupTable {
+    int32_t* tab;
+    const double *X, *Y;
+    unsigned size;
+    __device__ DupTable(const Batch& B, int64_t base, int n)
+        : tab(B.top_nbr + 2 * base), X(B.X_in + base), Y(B.Y_in + base), size(2u * (unsigned)n) {}
+    __device__ unsigned first(double x, double y) const {
+        unsigned long long h = (unsigned long long)__double_as_longlong(x + 0.0) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 32;
+        h = (h ^ (unsigned long long)__double_as_longlong(y + 0.0)) * 0xbf58476d1ce4e5b9ull;
+        h ^= h >> 29;
+        return (unsigned)(((h >> 32) * (unsigned long long)size) >> 32);
+    }
+    __device__ bool same(int j, double x, double y) const { return round3(X[j]) == x && round3(Y[j]) == y; }
+    __device__ void insert(int i, double x, double y) const {
+        unsigned h = first(x, y);
+        for (unsigned p = 0; p < size; ++p) {
+            const int cur = atomicCAS(tab + h, -1, i);
+            if (cur < 0) return;
+            if (same(cur, x, y)) { atomicMin(tab + h, i); return; }
+            if (++h == size) h = 0;
+        }
+    }
+    // the first point equal to point i (i itself when it is the first)
+    __device__ int find(int i, double x, double y) const {
+        unsigned h = first(x, y);
+        for (unsigned p = 0; p < size; ++p) {
+            const int cur = tab[h];
+            if (cur < 0) return i;
+            if (cur == i || same(cur, x, y)) return cur;
+            if (++h == size) h = 0;
+        }
+        return i;
+    }
+};
+__global__ void __launch_bounds__(kT) k_round(Batch B) {
+    const int c = blockIdx.x;
+    const int b = B.chunk_inst[c];
+    const int64_t base = B.offs[b];
+    const int n = (int)(B.offs[b + 1] - base);
+    const int i = B.chunk_start[c] + threadIdx.x;
+    if (i >= n) return;
+    const double x = round3(B.X_in[base + i]), y = round3(B.Y_in[base + i]);
+    B.Pr[base + i] = make_double2(x, y);
+    B.dup_of[base + i] = -1;
+    if (!B.skip_dedup) DupTable(B, base, n).insert(i, x, y);
+}
+__global__ void __launch_bounds__(kT) k_dup(Batch B) {
+    const int c = blockIdx.x;
+    const int b = B.chunk_inst[c];
+    const int64_t base = B.offs[b];
+    const int n = (int)(B.offs[b + 1] - base);
+    const int i = B.chunk_start[c] + threadIdx.x;
+    if (i >= n) return;
+    const double2 p = B.Pr[base + i];
+    const int j = DupTable(B, base, n).find(i, p.x, p.y);
+    if (j != i) B.dup_of[base + i] = j;
+}
+
+/* ------------------------------------------------------------------ */
+/* k_prep: compaction, bbox, cell grid (FXY.hpp:231-309)                 */
 /* ------------------------------------------------------------------ */
 __global__ void __launch_bounds__(kT) k_prep(Batch B) {
     const int b = blockIdx.x;
     const int64_t base = B.offs[b];
     const int n = (int)(B.offs[b + 1] - base);
-    __shared__ double2 tile[kTile];
     __shared__ int swarp[kT / 32 + 1];
     __shared__ int s_carry;
     __shared__ double sred[kT / 32];
-
-    for (int i = threadIdx.x; i < n; i += kT) {
-        B.Pr[base + i] = make_double2(round3(B.X_in[base + i]), round3(B.Y_in[base + i]));
-        B.dup_of[base + i] = -1;
-    }
-    __syncthreads();
-    // a point is dropped if an earlier point has identical rounded
-    // coordinates; it maps to the first such point (FXY.hpp:260-265)
-    for (int t0 = 0; t0 < n && !B.skip_dedup; t0 += kTile) {
-        const int cnt = min(kTile, n - t0);
-        for (int k = threadIdx.x; k < cnt; k += kT) tile[k] = B.Pr[base + t0 + k];
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += kT) {
-            if (i <= t0 || B.dup_of[base + i] >= 0) continue;
-            const double2 p = B.Pr[base + i];
-            const int jmax = min(cnt, i - t0);
-            for (int k = 0; k < jmax; ++k)
-                if (tile[k].x == p.x && tile[k].y == p.y) { B.dup_of[base + i] = t0 + k; break; }
-        }
-        __syncthreads();
-    }
     if (threadIdx.x == 0) s_carry = 0;
     __syncthreads();
-    for (int r = 0; r < n; r += kT) {
-        const int i = r + threadIdx.x;
-        const int keep = (i < n && B.dup_of[base + i] < 0) ? 1 : 0;
+    constexpr int kPer = 4;  // consecutive points of a thread in a round
+    for (int r = 0; r < n; r += kT * kPer) {
+        const int i0 = r + threadIdx.x * kPer;
+        int keep = 0;
+#pragma unroll
+        for (int c = 0; c < kPer; ++c)
+            if (i0 + c < n && B.dup_of[base + i0 + c] < 0) keep |= 1 << c;
         int tot;
-        const int ex = block_excl_scan<kT>(keep, swarp, &tot);
-        if (keep) {
-            const int id = s_carry + ex;
-            B.P[base + id] = B.Pr[base + i];
-            B.K[base + id] = B.K_in ? B.K_in[base + i] : i + 1;
-        }
+        int id = s_carry + block_excl_scan<kT>(__popc(keep), swarp, &tot);
+#pragma unroll
+        for (int c = 0; c < kPer; ++c)
+            if ((keep >> c) & 1) {
+                B.P[base + id] = B.Pr[base + i0 + c];
+                B.K[base + id] = B.K_in ? B.K_in[base + i0 + c] : i0 + c + 1;
+                ++id;
+            }
         __syncthreads();
         if (threadIdx.x == 0) s_carry += tot;
         __syncthreads();
@@ -203,7 +256,8 @@ __global__ void __launch_bounds__(kT) k_cutoff(Batch B) {
     const int N = min(B.N_cut, V - 1);  // FXY.hpp:77
     const double s = 2.0 * B.spn[b];    // FXY.hpp:78
     const int nx = B.gnx[b];
-    for (int qi = w; qi < kT && i0 + qi < V; qi += kT / 32) {
+    const int q1 = ((blockIdx.y + 1) * kT) / gridDim.y;  // this CTA's part of the chunk
+    for (int qi = (blockIdx.y * kT) / gridDim.y + w; qi < q1 && i0 + qi < V; qi += kT / 32) {
         const int i = i0 + qi;
         const double2 me = B.P[base + i];
         int L = 0, st = 0, passes = 0;
@@ -304,7 +358,8 @@ __global__ void __launch_bounds__(kT) k_select(Batch B) {
     const int nx = B.gnx[b];
     const int mode = B.cost_mode;
     const unsigned FULL = 0xffffffffu;
-    for (int qi = w; qi < kT && i0 + qi < V; qi += kT / 32) {
+    const int q1 = ((blockIdx.y + 1) * kT) / gridDim.y;  // this CTA's part of the chunk
+    for (int qi = (blockIdx.y * kT) / gridDim.y + w; qi < q1 && i0 + qi < V; qi += kT / 32) {
         const int i = i0 + qi;
         const double2 me = B.P[base + i];
         const double cut_i = B.cut[base + i];
@@ -1690,6 +1745,15 @@ cudaError_t launch_axb(const Batch& B, const DevParams& P, cudaStream_t s, int64
 /* host launchers                                                       */
 /* ------------------------------------------------------------------ */
 cudaError_t launch_prep(const Batch& B, cudaStream_t s, int64_t* launches) {
+    if (B.n_chunks > 0) {
+        if (!B.skip_dedup) {
+            cudaError_t e = cudaMemsetAsync(B.top_nbr, 0xff, sizeof(int32_t) * 2 * B.n_total, s);
+            if (e != cudaSuccess) return e;
+        }
+        k_round<<<B.n_chunks, kT, 0, s>>>(B);
+        if (!B.skip_dedup) k_dup<<<B.n_chunks, kT, 0, s>>>(B);
+        *launches += B.skip_dedup ? 1 : 2;
+    }
     k_prep<<<B.n_inst, kT, 0, s>>>(B);
     ++*launches;
     return cudaGetLastError();
@@ -1704,13 +1768,19 @@ cudaError_t launch_knn(const Batch& B, int64_t* scan_scratch, cudaStream_t s, in
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = launch_scan(B.cellcnt, B.cellstart, B.n_total, scan_scratch, s, launches)) != cudaSuccess) return e;
     k_grid_scatter<<<B.n_chunks, kT, 0, s>>>(B);
-    k_cutoff<<<B.n_chunks, kT, 0, s>>>(B);
+    // a warp takes the 32 nodes of a chunk's eighth one after the other; with few
+    // chunks they are spread over more CTAs, down to one node a warp (300 points:
+    // both kernels 0.43 -> 0.06 ms)
+    int parts = 1;
+    while (parts < 32 && (int64_t)B.n_chunks * parts < 2048) parts *= 2;
+    const dim3 grid(B.n_chunks, parts);
+    k_cutoff<<<grid, kT, 0, s>>>(B);
     *launches += 2;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (B.N <= 32) k_select<1><<<B.n_chunks, kT, 0, s>>>(B);
-    else if (B.N <= 64) k_select<2><<<B.n_chunks, kT, 0, s>>>(B);
-    else if (B.N <= 128) k_select<4><<<B.n_chunks, kT, 0, s>>>(B);
-    else k_select<8><<<B.n_chunks, kT, 0, s>>>(B);
+    if (B.N <= 32) k_select<1><<<grid, kT, 0, s>>>(B);
+    else if (B.N <= 64) k_select<2><<<grid, kT, 0, s>>>(B);
+    else if (B.N <= 128) k_select<4><<<grid, kT, 0, s>>>(B);
+    else k_select<8><<<grid, kT, 0, s>>>(B);
     ++*launches;
     return cudaGetLastError();
 }

@@ -150,7 +150,6 @@ DevParams to_dev(const f2m_params& p) {
 /* batch plan + device layout                                           */
 /* ------------------------------------------------------------------ */
 constexpr int kChunk = 256;
-constexpr int32_t kHostDedupPoints = 16384;
 
 struct Plan {
     int32_t n_inst = 0;
@@ -415,49 +414,6 @@ void parallel_sort(std::vector<T>& a, Less less, int64_t serial_below = 200000) 
             });
         for (auto& th : pool) th.join();
         a.swap(tmp);
-    }
-}
-
-// get_KXY's rounding and de-duplication (FXY.hpp:252-267): coordinates
-// rounded to 1e-3 and the first occurrence of each rounded point kept, in
-// input order.  A sort of the rounded points (ties by input index) finds the
-// repeats instead of the reference's nested hash maps; +0 and -0 compare
-// equal and a point with a NaN coordinate is never a repeat, as there.
-void host_dedup_points(const double* x, const double* y, const int32_t* labels, int32_t n,
-                       std::vector<double>& hx, std::vector<double>& hy, std::vector<int32_t>& hl) {
-    std::vector<double> rx(n), ry(n);
-    parallel_for(n, [&](int64_t i0, int64_t i1) {
-        for (int64_t i = i0; i < i1; ++i) {
-            double xx = std::round(x[i] * 1000), yy = std::round(y[i] * 1000);
-            rx[i] = xx / 1000;
-            ry[i] = yy / 1000;
-        }
-    });
-    auto nanp = [&](int32_t i) { return rx[i] != rx[i] || ry[i] != ry[i]; };
-    std::vector<int32_t> idx(n);
-    for (int32_t i = 0; i < n; ++i) idx[i] = i;
-    parallel_sort(idx, [&](int32_t a, int32_t b) {
-        const bool na = nanp(a), nb = nanp(b);
-        if (na != nb) return nb;
-        if (!na) {
-            if (rx[a] != rx[b]) return rx[a] < rx[b];
-            if (ry[a] != ry[b]) return ry[a] < ry[b];
-        }
-        return a < b;
-    }, 50000);
-    std::vector<char> dup(n, 0);
-    for (int32_t k = 1; k < n; ++k) {
-        const int32_t a = idx[k - 1], b = idx[k];
-        if (!nanp(a) && !nanp(b) && rx[a] == rx[b] && ry[a] == ry[b]) dup[b] = 1;
-    }
-    hx.clear();
-    hy.clear();
-    hl.clear();
-    for (int32_t i = 0; i < n; ++i) {
-        if (dup[i]) continue;
-        hx.push_back(rx[i]);
-        hy.push_back(ry[i]);
-        hl.push_back(labels ? labels[i] : i + 1);
     }
 }
 
@@ -1640,24 +1596,9 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     if (params) prm = *params;
     cudaSetDevice(ctx->device);
     std::unique_ptr<f2m_result> R(new f2m_result());
-    // Large inputs are rounded and de-duplicated on the host, as get_KXY does
-    // (FXY.hpp:252-267); the device's per-instance pass is quadratic.
-    std::vector<double> hx, hy;
-    std::vector<int32_t> hl;
-    bool host_dedup = n > kHostDedupPoints;
     StageClock clk;
-    if (host_dedup) {
-        host_dedup_points(x, y, labels, n, hx, hy, hl);
-        x = hx.data();
-        y = hy.data();
-        labels = hl.data();
-        n = (int32_t)hx.size();
-    }
-    clk.mark("dedup");
-    const int64_t offs2[2] = {0, n};
     DevCall C;
-    if ((s = setup_call(ctx, C, 1, offs2, top_k, prm, true))) return s;
-    C.B.skip_dedup = host_dedup ? 1 : 0;
+    if ((s = setup_call(ctx, C, 1, offs, top_k, prm, true))) return s;
     int32_t* dK = nullptr;
     if (labels) {
         // labels ride in the (unused) cursor buffer until k_prep compacts them
@@ -1665,7 +1606,7 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
         C.B.K_in = dK;
         F2M_CUDA(cudaMemcpyAsync(dK, labels, n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     }
-    F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(C.B.offs), offs2, 2 * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(C.B.offs), offs, 2 * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.X_in), x, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.Y_in), y, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     auto t0 = std::chrono::steady_clock::now();
