@@ -1311,46 +1311,64 @@ cudaError_t launch_grid_order(const Batch& B, const GridState& G, int b, int V, 
 /* ------------------------------------------------------------------ */
 /* the reference's edge order of one instance                           */
 /* ------------------------------------------------------------------ */
-// Per slot of node v: keys (emitter << 32 | partner) and the cost's bits
-// (costs are non-negative, so their bits order as the values) for a slot
-// whose neighbour is the higher id, all ones (last) otherwise.
-__global__ void k_edge_keys(Batch B, int b, int V, unsigned long long* k1, uint32_t* v1) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V) return;
+// The slots whose neighbour is the higher id (each edge once), packed in any
+// order (*count of them): the key emitter * V + partner, which no two edges
+// share, so the sorted order does not depend on the packing.
+__global__ void k_edge_keys(Batch B, int b, int V, unsigned long long* k1, uint32_t* v1, unsigned* count) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const int64_t base = B.offs[b];
     const int64_t s0 = B.row[base];
-    for (int64_t a = B.row[base + v]; a < B.row[base + v + 1]; ++a) {
-        const bool up = B.slot[a].nbr > v;
-        k1[a - s0] = up ? (((unsigned long long)(unsigned)B.s_em[a] << 32) | (unsigned)B.s_oth[a]) : ~0ull;
-        v1[a - s0] = (uint32_t)(a - s0);
+    const int64_t r0 = v < V ? B.row[base + v] : 0, r1 = v < V ? B.row[base + v + 1] : 0;
+    int c = 0;
+    for (int64_t a = r0; a < r1; ++a) c += B.slot[a].nbr > v;
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    unsigned at = 0;
+    if (lane == 31) at = atomicAdd(count, (unsigned)inc);
+    at = __shfl_sync(0xffffffffu, at, 31) + inc - c;
+    for (int64_t a = r0; a < r1; ++a) {
+        if (B.slot[a].nbr <= v) continue;
+        k1[at] = (unsigned long long)(unsigned)B.s_em[a] * (unsigned)V + (unsigned)B.s_oth[a];
+        v1[at] = (uint32_t)(a - s0);
+        ++at;
     }
 }
-__global__ void k_edge_cost_keys(Batch B, int b, int64_t S, const unsigned long long* k1, const uint32_t* v1,
-                                 unsigned long long* k2) {
+// the costs' bits (costs are non-negative, so their bits order as the values)
+__global__ void k_edge_cost_keys(Batch B, int b, int64_t E, const uint32_t* v1, unsigned long long* k2) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t s0 = B.row[B.offs[b]];
-    k2[i] = k1[i] == ~0ull ? ~0ull : (unsigned long long)__double_as_longlong(B.s_cost[s0 + v1[i]]);
+    if (i >= E) return;
+    k2[i] = (unsigned long long)__double_as_longlong(B.s_cost[B.row[B.offs[b]] + v1[i]]);
 }
 
 size_t edge_order_temp_bytes(int64_t S) { return radix_sort_temp_bytes(S); }
 
 cudaError_t launch_edge_order(const Batch& B, int b, int V, int64_t S, const EdgeSort& E, const uint32_t** order,
                               cudaStream_t s, int64_t* launches) {
-    if (V <= 0 || S <= 0) { *order = E.v2; return cudaSuccess; }
+    const int64_t n = S / 2;
+    if (V <= 0 || n <= 0) { *order = E.v2; return cudaSuccess; }
     const int T = 256;
-    k_edge_keys<<<(V + T - 1) / T, T, 0, s>>>(B, b, V, E.k1, E.v1);
+    unsigned* count = static_cast<unsigned*>(E.xout);  // free until the export
+    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    k_edge_keys<<<(V + T - 1) / T, T, 0, s>>>(B, b, V, E.k1, E.v1, count);
     ++*launches;
-    // LSD: by (emitter, partner), then stably by cost
+    // LSD: by (emitter, partner), over the bits that V * V takes, then stably by
+    // cost
+    int bits = 1;
+    while (bits < 62 && ((unsigned long long)V * (unsigned)V >> bits) != 0) ++bits;
     unsigned long long* ks = nullptr;
     uint32_t* vs = nullptr;
-    cudaError_t e = radix_sort(E.k1, E.k2, E.v1, E.v2, S, 0, 64, E.tmp, E.tmp_bytes, s, launches, &ks, &vs);
+    e = radix_sort(E.k1, E.k2, E.v1, E.v2, n, 0, bits, E.tmp, E.tmp_bytes, s, launches, &ks, &vs);
     if (e != cudaSuccess) return e;
     unsigned long long* kc = (ks == E.k1) ? E.k2 : E.k1;  // the free key buffer
     uint32_t* vfree = (vs == E.v1) ? E.v2 : E.v1;
-    k_edge_cost_keys<<<(unsigned)((S + T - 1) / T), T, 0, s>>>(B, b, S, ks, vs, kc);
+    k_edge_cost_keys<<<(unsigned)((n + T - 1) / T), T, 0, s>>>(B, b, n, vs, kc);
     ++*launches;
-    e = radix_sort(kc, ks, vs, vfree, S, 0, 64, E.tmp, E.tmp_bytes, s, launches, &ks, &vs);
+    e = radix_sort(kc, ks, vs, vfree, n, 0, 64, E.tmp, E.tmp_bytes, s, launches, &ks, &vs);
     if (e != cudaSuccess) return e;
     *order = vs;
     return cudaGetLastError();
@@ -1400,6 +1418,32 @@ __global__ void k_export_edges(Batch B, int b, int V, const uint32_t* order, int
         X.D[e] = s.D;
         X.x[e] = c == 3 ? (double)B.xval[a] : (c == 2 ? 1.0 : (c == 1 ? 0.5 : 0.0));
     }
+}
+
+// The scalars of one solved instance, for one copy to the host.
+__global__ void k_pack_result(Batch B, int b, ResultPack* p) {
+    ResultPack r;
+    r.base = B.offs[b];
+    r.V = B.Vn[b];
+    r.status = B.status[b];
+    r.dmin_bits = B.dmin_bits[b];
+    r.n_combs = B.n_combs[b];
+    r.n_irr = B.n_irr[b];
+    r.max_rank = B.max_rank[b];
+    r.deg_viol = B.deg_viol[b];
+    r.checks = B.checks[b];
+    r.lp = B.lp[b];
+    r.dual = B.dual[b];
+    r.max_grad = B.max_grad[b];
+    r.iters = B.iters[b];
+    r.r0 = B.row[r.base];
+    r.r1 = B.row[r.base + r.V];
+    *p = r;
+}
+cudaError_t launch_pack_result(const Batch& B, int b, ResultPack* p, cudaStream_t s, int64_t* launches) {
+    k_pack_result<<<1, 1, 0, s>>>(B, b, p);
+    ++*launches;
+    return cudaGetLastError();
 }
 
 cudaError_t launch_export_edges(const Batch& B, int b, int V, const uint32_t* order, int64_t E,

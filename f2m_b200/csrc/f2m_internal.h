@@ -187,12 +187,20 @@ struct EdgeExport {
     double *Do, *D, *x;
 };
 EdgeExport edge_export_view(void* xout, int64_t E);
+// What the host needs of a solved instance before its arrays.
+struct ResultPack {
+    int64_t base, r0, r1, iters;
+    unsigned long long dmin_bits;
+    double lp, dual, max_grad;
+    int32_t V, status, n_combs, n_irr, max_rank, deg_viol, checks;
+};
+cudaError_t launch_pack_result(const Batch& B, int b, ResultPack* p, cudaStream_t s, int64_t* launches);
 cudaError_t launch_export_edges(const Batch& B, int b, int V, const uint32_t* order, int64_t E,
                                 const EdgeExport& X, cudaStream_t s, int64_t* launches);
 // The reference's edge order (ascending cost, then emitter, then partner:
 // graph_tour.hpp:28-98) of instance b's edges, each as the offset of its slot
-// in the lower-id endpoint's list (within the instance's slots); the first
-// S/2 entries of *order are the edges in order.
+// in the lower-id endpoint's list (within the instance's slots); the S/2
+// entries of *order are the edges in order.
 cudaError_t launch_edge_order(const Batch& B, int b, int V, int64_t S, const EdgeSort& E, const uint32_t** order,
                               cudaStream_t s, int64_t* launches);
 // FP64 pipe throughput probe (f2m_probe.cu): kind 0 DADD chains, kind 1 DSETP.

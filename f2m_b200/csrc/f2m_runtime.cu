@@ -767,7 +767,7 @@ void carve_edge_sort(Arena& A, EdgeSort& E, int64_t S) {
     E.v2 = A.take<uint32_t>(S);
     E.tmp_bytes = edge_order_temp_bytes(S);
     E.tmp = A.take<unsigned char>(E.tmp_bytes);
-    E.xout = A.take<double>((S * 20 + 7) / 8);  // E = S/2 edges x 40 bytes
+    E.xout = A.take<double>(std::max<int64_t>((S * 20 + 7) / 8, 32));  // E = S/2 edges x 40 bytes (or a ResultPack)
 }
 
 // A single instance above this many points runs on the whole GPU although one
@@ -1095,32 +1095,16 @@ f2m_status complete_instance(f2m_ctx* ctx, DevCall& C, int b, const f2m_params& 
 // rounding).  The host builds none of the comb stage's structures.  Used by
 // the points path; the file path keeps the host stage, which also writes the
 // reference's files.
-f2m_status export_from_device(f2m_ctx* ctx, const DevCall& C, int b, f2m_result& R) {
+f2m_status export_from_device(f2m_ctx* ctx, const DevCall& C, int b, const ResultPack& rp, f2m_result& R) {
     Range rg("f2m export instance (device)");
     const Batch& B = C.B;
     HostInst& H = R.H;
-    int32_t V = 0, nc = 0, ni = 0, mr = 0, viol = 0;
-    int64_t base = 0;
-    unsigned long long db = 0;
-    double lp = 0, dual = 0;
+    const int32_t V = rp.V;
+    const int64_t base = rp.base;
     auto small = [&](void* dst, const void* src, size_t n) {
         return cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, ctx->stream);
     };
-    F2M_CUDA(small(&V, B.Vn + b, 4));
-    F2M_CUDA(small(&base, B.offs + b, 8));
-    F2M_CUDA(small(&db, B.dmin_bits + b, 8));
-    F2M_CUDA(small(&nc, B.n_combs + b, 4));
-    F2M_CUDA(small(&ni, B.n_irr + b, 4));
-    F2M_CUDA(small(&mr, B.max_rank + b, 4));
-    F2M_CUDA(small(&viol, B.deg_viol + b, 4));
-    F2M_CUDA(small(&lp, B.lp + b, 8));
-    F2M_CUDA(small(&dual, B.dual + b, 8));
-    F2M_CUDA(cudaStreamSynchronize(ctx->stream));
-    int64_t r0 = 0, r1 = 0;
-    F2M_CUDA(small(&r0, B.row + base, 8));
-    F2M_CUDA(small(&r1, B.row + base + V, 8));
-    F2M_CUDA(cudaStreamSynchronize(ctx->stream));
-    const int64_t S = r1 - r0, E = S / 2;
+    const int64_t S = rp.r1 - rp.r0, E = S / 2;
     const uint32_t* ord = nullptr;
     F2M_CUDA(launch_edge_order(B, b, V, S, C.es, &ord, ctx->stream, &ctx->launches));
     const EdgeExport X = edge_export_view(C.es.xout, E);
@@ -1137,7 +1121,7 @@ f2m_status export_from_device(f2m_ctx* ctx, const DevCall& C, int b, f2m_result&
     const EdgeExport P = edge_export_view(q, E);
     H.V = V;
     H.E = (int)E;
-    std::memcpy(&H.dmin, &db, sizeof(double));
+    std::memcpy(&H.dmin, &rp.dmin_bits, sizeof(double));
     H.label.assign(K, K + V);
     H.F.assign(F, F + V);
     H.ev1.resize(E); H.ev2.resize(E); H.el1.resize(E); H.el2.resize(E);
@@ -1153,16 +1137,19 @@ f2m_status export_from_device(f2m_ctx* ctx, const DevCall& C, int b, f2m_result&
         std::memcpy(R.x.data() + e0, P.x + e0, n8);
     });
     R.X.clear();
-    R.lp = lp;
-    R.max_rank = mr;
+    R.lp = rp.lp;
+    R.max_rank = rp.max_rank;
     R.status = F2M_OK;
     R.st.repair_steps = 0;
-    R.st.irr_a = ni;  // irregular combs, solved by Ax=b on the device
+    R.st.irr_a = rp.n_irr;  // irregular combs, solved by Ax=b on the device
     R.st.irr_b = 0;
-    R.st.n_combs = nc;
-    R.st.degree_violations = viol;
-    R.st.dual_value = dual;
+    R.st.n_combs = rp.n_combs;
+    R.st.degree_violations = rp.deg_viol;
+    R.st.dual_value = rp.dual;
     R.st.d_min = H.dmin;
+    R.st.iterations = rp.iters;
+    R.st.checks = rp.checks;
+    R.st.max_grad = rp.max_grad;
     return F2M_OK;
 }
 
@@ -1646,9 +1633,15 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     F2M_CUDA(cudaEventRecord(ctx->ev[4], ctx->stream));
     ctx->timed = true;
     ctx->last = C.B;
-    int32_t st = 0;
-    F2M_CUDA(cudaMemcpyAsync(&st, C.B.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+    // the scalars of the result in one copy (the export buffer is free until then)
+    ResultPack* pack = static_cast<ResultPack*>(C.es.xout);
+    F2M_CUDA(launch_pack_result(C.B, 0, pack, ctx->stream, &ctx->launches));
+    F2M_CUDA(ensure_pinned(ctx, sizeof(ResultPack)));
+    F2M_CUDA(cudaMemcpyAsync(ctx->pinned, pack, sizeof(ResultPack), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    ResultPack rp;
+    std::memcpy(&rp, ctx->pinned, sizeof(rp));
+    const int32_t st = rp.status;
     clk.mark("device");
     if (st != F2M_OK && st != kNeedsHost) {
         R->status = st;
@@ -1665,7 +1658,7 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     // otherwise (an Ax=b system that did not converge, so the repair loop
     // runs) the host comb stage as the reference runs it
     if (st == F2M_OK) {
-        if ((s = export_from_device(ctx, C, 0, *R))) return s;
+        if ((s = export_from_device(ctx, C, 0, rp, *R))) return s;
         clk.mark("export");
     } else {
         if ((s = pull_instance(ctx, C, 0, R->H, true))) return s;
@@ -1673,7 +1666,7 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
         if ((s = complete_instance(ctx, C, 0, prm, *R))) return s;
     }
     clk.mark("complete");
-    if ((s = pull_stats(ctx, C, 0, *R))) return s;
+    if (st != F2M_OK && (s = pull_stats(ctx, C, 0, *R))) return s;
     R->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     *out = R.release();
     return (f2m_status)(*out)->status;

@@ -88,6 +88,43 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned long l
     }
 }
 
+// Exclusive scan of up to kScanOne counts by one CTA, a contiguous run of them
+// per thread: one launch a pass where the general scan takes three and a copy
+// (a pass over 2,000 keys is launches, not work).
+constexpr int kScanOne = 65536;
+__global__ void __launch_bounds__(1024) k_rs_scan(const int64_t* in, int64_t* out, int n) {
+    __shared__ long long swarp[32];
+    const int per = (n + 1023) / 1024, b0 = threadIdx.x * per, b1 = min(n, b0 + per);
+    long long sum = 0;
+    for (int k = b0; k < b1; ++k) sum += in[k];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    long long inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) swarp[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+        const long long x = swarp[lane];
+        long long s = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += y;
+        }
+        swarp[lane] = s - x;
+    }
+    __syncthreads();
+    long long run = swarp[w] + inc - sum;
+    for (int k = b0; k < b1; ++k) {
+        const long long c = in[k];
+        out[k] = run;
+        run += c;
+    }
+}
+
 size_t radix_sort_temp_bytes(int64_t n) {
     const int64_t cells = 256 * std::max<int64_t>(rs_tiles(n), 1);
     return (size_t)(2 * cells + scan_scratch_elems(cells) + 2) * sizeof(int64_t);
@@ -114,8 +151,13 @@ cudaError_t radix_sort(unsigned long long* keys, unsigned long long* kbuf, uint3
     for (int shift = begin_bit; shift < end_bit; shift += 8) {
         k_rs_hist<<<(unsigned)tiles, kRsThreads, 0, s>>>(ki, n, shift, tiles, count);
         ++*launches;
-        cudaError_t e = launch_scan(count, offset, cells, scratch, s, launches);
-        if (e != cudaSuccess) return e;
+        cudaError_t e = cudaSuccess;
+        if (cells <= kScanOne) {
+            k_rs_scan<<<1, 1024, 0, s>>>(count, offset, (int)cells);
+            ++*launches;
+        } else if ((e = launch_scan(count, offset, cells, scratch, s, launches)) != cudaSuccess) {
+            return e;
+        }
         if (vals) k_rs_scatter<true><<<(unsigned)tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, shift, tiles, offset);
         else k_rs_scatter<false><<<(unsigned)tiles, kRsThreads, 0, s>>>(ki, nullptr, ko, nullptr, n, shift, tiles, offset);
         ++*launches;
