@@ -870,19 +870,27 @@ struct TeamMem {
     int cap;
     int gcap;
     int NS;
+    bool whole;      // Ha and Hb have 32*NS places (else V: the potentials stay in node order)
 };
 constexpr int kSelGlobal = -(1 << 30);  // soff in [kSelGlobal, -1]: global SELL
 constexpr int kSelNode = INT_MIN;
 
 __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+__device__ __host__ inline size_t team_fixed_bytes(int V) {
+    const int NS = (V + 31) / 32;
+    return (size_t)V * 16 + (size_t)NS * 8 + 258 * 4 + (size_t)NS * 64 + 5 * 16;
+}
 __device__ __forceinline__ TeamMem carve_team(unsigned char* base, size_t bytes, const Batch& B, int b,
                                               int V) {
     TeamMem M;
     M.NS = (V + 31) / 32;
     size_t o = 0;
-    M.Ha = reinterpret_cast<double*>(base + o); o += (size_t)M.NS * 32 * 8;
-    M.Hb = reinterpret_cast<double*>(base + o); o += (size_t)M.NS * 32 * 8;
+    // whole slices of potentials, where the share holds them
+    M.whole = team_fixed_bytes(32 * M.NS) <= bytes;
+    const size_t pots = (size_t)(M.whole ? 32 * M.NS : V) * 8;
+    M.Ha = reinterpret_cast<double*>(base + o); o += pots;
+    M.Hb = reinterpret_cast<double*>(base + o); o = align16(o + pots);
     M.soff = reinterpret_cast<int*>(base + o); o = align16(o + (size_t)M.NS * 4);
     M.swid = reinterpret_cast<int*>(base + o); o = align16(o + (size_t)M.NS * 4);
     M.hist = reinterpret_cast<int*>(base + o); o = align16(o + 258 * 4);
@@ -900,10 +908,6 @@ __device__ __forceinline__ TeamMem carve_team(unsigned char* base, size_t bytes,
     M.gcap = (int)(gcap < ((int64_t)1 << 29) ? gcap : ((int64_t)1 << 29));
     M.cnt = B.efcnt + p0;
     return M;
-}
-__device__ __host__ inline size_t team_fixed_bytes(int V) {
-    const int NS = (V + 31) / 32;
-    return (size_t)NS * 32 * 16 + (size_t)NS * 8 + 258 * 4 + (size_t)NS * 64 + 5 * 16;
 }
 
 __device__ __forceinline__ uint16_t ef_word(int v, int nbr) {
@@ -1213,7 +1217,6 @@ struct Solver {
     int checks = 0;
     bool capped = false;
     bool plain = false;     // magnitudes allow the short step forms (step_cost_plain)
-    bool node_lists = false;  // some slice is read from the node-indexed copy
     bool sliced = false;      // the potentials are in slice order
 
     __device__ Solver(const Batch& b, const DevParams& p, const Inst& i, const Team<TEAM>& t, TeamMem m)
@@ -1387,7 +1390,7 @@ struct Solver {
         }
         if (T.tid == 0) M.hist[257] = carry;  // read after the barriers below
         lead = T.max_ll(lead);
-        node_lists = carry - lead > M.gcap;
+        const bool by_node = carry - lead > M.gcap || !M.whole;  // (a slice in neither place, or no room)
         for (int s = T.tid; s < M.NS; s += TEAM) {
             const int pos = M.soff[s], size = 32 * M.swid[s];
             if (pos + size <= M.cap) continue;
@@ -1403,10 +1406,10 @@ struct Solver {
             uint16_t* dW = (off >= 0) ? M.eW + off : M.gsW + (off - kSelGlobal);
             const int v = (int)M.ord[s * 32 + lane];
             const int64_t go = I.row[v] - row0;
-            fill_slice_lane(I.gD + go, I.gN + go, node_lists ? nullptr : pos, M.cnt[v], M.swid[s], dD + lane, dW + lane);
+            fill_slice_lane(I.gD + go, I.gN + go, by_node ? nullptr : pos, M.cnt[v], M.swid[s], dD + lane, dW + lane);
         }
         T.sync();
-        if (node_lists) return;
+        if (by_node) return;
         for (int p = T.tid; p < 32 * M.NS; p += TEAM) Hn[p] = Hc[M.ord[p]];
         T.sync();
         swap_f();

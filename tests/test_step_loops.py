@@ -61,3 +61,32 @@ def test_potentials_on_one_sm_and_on_all(ctx, oracle, n, solver):
     assert np.array_equal(r.F, o.F)
     lp, st = ctx.solve_batch(np.array([0, n]), x, y, 10, params=f2m_b200.default_params(solver=solver))
     assert st[0] == o.status and abs(lp[0] - o.lp) <= 1e-12 * o.lp
+
+
+def test_largest_instance_of_a_class(ctx, oracle):
+    """The largest instance a 128-thread team's share of shared memory holds: its
+    last slice is cut short, so its potentials stay in node order."""
+    start = f2m_b200.get_class_bounds()
+    lo, hi = 4, 8000
+    try:
+        while lo < hi:
+            mid = (lo + hi + 1) // 2
+            try:
+                f2m_b200.set_class_bounds([mid, mid + 1, mid + 2])
+                lo = mid
+            except f2m_b200.F2MError:
+                hi = mid - 1
+        f2m_b200.set_class_bounds([lo, lo + 1, lo + 2])
+        x, y = synth.uniform_int_points(lo, 77)
+        o = oracle.solve_points(x, y, 6)
+        # enough instances that the call keeps the narrow teams; the others are small
+        sizes = np.array([lo] * 4 + [8] * 700, np.int64)
+        offs = np.concatenate([[0], np.cumsum(sizes)])
+        sx, sy = synth.uniform_int_points(8, 78)
+        X = np.concatenate([np.tile(x, 4), np.tile(sx, 700)])
+        Y = np.concatenate([np.tile(y, 4), np.tile(sy, 700)])
+        out = ctx.solve_batch(offs, X, Y, 6, details=True)
+        assert np.all(out["status"] == 0)
+        assert np.all(np.abs(out["lp"][:4] - o.lp) <= 1e-12 * o.lp)
+    finally:
+        f2m_b200.set_class_bounds(start)
