@@ -1933,10 +1933,24 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     const int32_t nck = std::max(1, (sp.iters + K - 1) / K);
     const int64_t S = 2 * n * N + 8 * n;  // union lists: own N + reverse (+ slack)
     // Under two instances an SM a pass of one CTA waits on its own latency and
-    // the whole GPU takes each pass instead: 200 instances of 200-1,200 points
-    // 15.1 ms (one CTA each) / 15.7 ms (a launch a pass) at tau 1e-3, 80 / 27 at
-    // 5e-2; 500 of 200-2,000 points 29 / 59 and 138 / 96.
-    const bool steps = sp.solver == 2 || (sp.solver == 0 && n_inst < 2 * ctx->sms);
+    // the whole GPU takes each pass instead.  So it does where tau is large
+    // against the point spacing (of the largest instance): whole lists are then
+    // within reach of a root (50 tau), more than a lane's scratch holds, and the
+    // lanes of a group share them.  Bound and gradient, 40 steps, one CTA each / a
+    // launch a pass, unit spacing: 600 instances of 100-500 points (N = 12) 7.0 /
+    // 9.0 ms at tau 1e-2, 18 / 9.9 at 5e-2; 600 of 200-1,500 (N = 28) 20.6 / 32.1
+    // and 65 / 44.
+    bool steps = sp.solver == 2;
+    if (sp.solver == 0) {
+        int32_t big = 0;
+        for (int32_t b = 1; b < n_inst; ++b)
+            if (offs[b + 1] - offs[b] > offs[big + 1] - offs[big]) big = b;
+        const auto bx = std::minmax_element(x + offs[big], x + offs[big + 1]);
+        const auto by = std::minmax_element(y + offs[big], y + offs[big + 1]);
+        const double w = (double)*bx.second - *bx.first, h = (double)*by.second - *by.first;
+        const double spacing = std::sqrt(w * h / (double)(offs[big + 1] - offs[big]));
+        steps = n_inst < 2 * ctx->sms || 50 * sp.tau > spacing;
+    }
     std::vector<int64_t> sbase(n_inst + 1, 0);  // slices, or warps of the per-step kernels
     const int64_t npw = smooth_nodes_per_warp(steps, n);
     std::vector<int32_t> order(n_inst);

@@ -1124,7 +1124,7 @@ int32_t smooth_max_nodes() {
 }
 
 // Rate of the logistic term at full occupancy: every thread accumulates four
-// independent LogitAcc sums (one exp and two divisions per term, the unit the
+// independent LogitAcc sums (one exp and one division per term, the unit the
 // persistent kernel counts), its arguments moving by a small step each round
 // so that nothing is loop-invariant.
 constexpr int kLogitProbeThreads = 256;
@@ -1162,8 +1162,10 @@ cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaSt
     cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     // two potential arrays, and a thread's scratch where it fits (an instance
     // near the limit re-reads its lists instead)
-    const size_t pot = (size_t)max_v * 16;
-    const int cap = (int)std::min<size_t>(kBuf, ((size_t)lim - 1024 - pot) / (kST * 10));
+    const size_t pot = (size_t)max_v * 16, room = (size_t)lim - 1024;
+    const size_t half = room / 2 - 1024;  // of two CTAs on an SM
+    const size_t fit = pot + kBuf * kST * 10 <= half ? half : room;
+    const int cap = (int)std::min<size_t>(fit == half ? 2 * kBuf : kBuf, (fit - pot) / (kST * 10));
     const size_t dyn = pot + (size_t)cap * kST * 10;
     const void* fn = grad ? (const void*)k_sbound<true> : (const void*)k_sbound<false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
