@@ -45,17 +45,16 @@ FLUSH_BYTES = 256 << 20
 LP_TOL = 1e-9
 
 # FP64 pipe operations of the persistent solver's Jacobi step, counted from
-# its source (f2m_kernels.cu Solver::step / slice_hgrad / half_grad,
-# f2m_device.cuh top3_insert):
+# its source (f2m_kernels.cu step_slices / step_one, f2m_device.cuh mid_sum):
 #   per list entry a warp lane sweeps (padding of the 32-node slices
-#   included): 2 DADD for the reduced cost (D + H[lo]) + H[hi] and 3 DSETP
-#   for the top-3 insertion;
-#   per lane updating a node: 1 DSETP (first value below the 1e6 sentinels),
-#   1 DADD (v1 + v2), 2 DMUL (/2, *0.5) and 1 DADD (H + grad/2).
+#   included): 2 DADD for the reduced cost (D + H[lo]) + H[hi] and at least
+#   one DSETP of the selection network (two for three entries, four for four,
+#   and two or three against the 1e6 sentinels);
+#   per lane updating a node: 1 DADD (v1 + v2) and 1 DFMA (H - (v1 + v2) / 4).
 # Partitions, gradient checks and comb extraction are not counted, so the
 # fraction is a lower bound.
-FP64_PER_ENTRY = 5
-FP64_PER_LANE = 5
+FP64_PER_ENTRY = 3
+FP64_PER_LANE = 2
 
 
 def parse():
@@ -593,10 +592,12 @@ def smooth_sub(args, local_rank, steps=3, warmup=1):
         kms.append(km)
     clocks = clk.stop()
     launches = ctx.kernel_launches() - l0
-    # roofline: the persistent kernel (one CTA per instance) evaluates
-    # logistic terms (one FP64 exp and two divisions each: the Newton sums
-    # of every node root, softplus, sigma and sigma'); its peak is the same
-    # term measured at full occupancy on this GPU
+    # the persistent kernel's rate of logistic terms (one FP64 exp and one
+    # division each: the Newton sums of every node root, softplus, sigma and
+    # sigma') beside the rate of evaluating each of them, measured at full
+    # occupancy on this GPU.  The sums cover every list entry; entries out of
+    # reach of the root are counted and not evaluated, so the ratio is no
+    # fraction of a peak and may pass 1.
     peak_terms = ctx.fp64_rate(2, repeats=3)
     ctx.close()
     t = float(np.mean(ms))
@@ -619,6 +620,8 @@ def smooth_sub(args, local_rank, steps=3, warmup=1):
                      "peak_kind": "measured in this run (f2m_fp64_rate kind 2: the same term, four "
                                   "independent sums per thread, every SM at full occupancy)",
                      "terms_per_launch": float(np.mean(kterms)), "kernel_ms": float(np.mean(kms)),
+                     "terms": "list entries the sums cover; those out of reach of the root are "
+                              "counted and not evaluated",
                      "traffic": None},
     }
     if not args.no_cpu_baseline:

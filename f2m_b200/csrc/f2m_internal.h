@@ -280,7 +280,7 @@ struct SmoothBatch {
     float* gx = nullptr;                // [n_total]
     float* gy = nullptr;                // [n_total]
     int32_t* queue = nullptr;
-    unsigned long long* work = nullptr; // [1] logistic terms evaluated by the persistent kernel
+    unsigned long long* work = nullptr; // [1] logistic terms covered by the persistent kernel
 };
 cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStream_t s,
                                 int64_t* launches);
@@ -289,8 +289,8 @@ cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaSt
 cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches);
 int32_t smooth_max_nodes();
 int smooth_nodes_per_warp(bool steps, int64_t n_total);
-// Rate probe of the smoothed bound's logistic term (one exp and two
-// divisions, the Newton sums' unit of work), and its work per launch.
+// Rate probe of the smoothed bound's logistic term (one exp and one division,
+// the Newton sums' unit of work), and its work per launch.
 cudaError_t launch_logit_probe(int blocks, int iters, double* out, cudaStream_t s);
 double logit_probe_terms(int blocks, int iters);
 
