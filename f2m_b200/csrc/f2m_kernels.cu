@@ -46,8 +46,10 @@ __device__ __forceinline__ double round3(double x) {
 // two places a point (in top_nbr, free until the kNN) holds point indices; equal
 // points meet in one place, which keeps the smallest index, and a second kernel
 // reads it back.  +0 and -0 are equal, NaN equals nothing, as in the
-// comparison.  (Thread per point over the whole GPU: 5,000 points took 2.65 ms
-// as a quadratic pass of one CTA, 100,000 took 4.5 ms as a sort on the host.)
+// comparison; points with a NaN stay out of the table, where those of the same
+// bits would share one start and probe past each other.  (Thread per point over
+// the whole GPU: 5,000 points took 2.65 ms as a quadratic pass of one CTA,
+// 100,000 took 4.5 ms as a sort on the host.)
 struct DupTable {
     int32_t* tab;
     const double *X, *Y;
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(kT) k_round(Batch B) {
     const double x = round3(B.X_in[base + i]), y = round3(B.Y_in[base + i]);
     B.Pr[base + i] = make_double2(x, y);
     B.dup_of[base + i] = -1;
-    if (!B.skip_dedup) DupTable(B, base, n).insert(i, x, y);
+    if (!B.skip_dedup && x == x && y == y) DupTable(B, base, n).insert(i, x, y);
 }
 __global__ void __launch_bounds__(kT) k_dup(Batch B) {
     const int c = blockIdx.x;
@@ -103,6 +105,7 @@ __global__ void __launch_bounds__(kT) k_dup(Batch B) {
     const int i = B.chunk_start[c] + threadIdx.x;
     if (i >= n) return;
     const double2 p = B.Pr[base + i];
+    if (p.x != p.x || p.y != p.y) return;
     const int j = DupTable(B, base, n).find(i, p.x, p.y);
     if (j != i) B.dup_of[base + i] = j;
 }
@@ -260,6 +263,11 @@ __global__ void __launch_bounds__(kT) k_cutoff(Batch B) {
     for (int qi = (blockIdx.y * kT) / gridDim.y + w; qi < q1 && i0 + qi < V; qi += kT / 32) {
         const int i = i0 + qi;
         const double2 me = B.P[base + i];
+        // no point is within any radius of a NaN: the passes below would end so too
+        if (me.x != me.x || me.y != me.y) {
+            if (lane == 0) B.status[b] = F2M_ERR_CAPACITY;
+            continue;
+        }
         int L = 0, st = 0, passes = 0;
         double cut = 0.0;
         for (;;) {
