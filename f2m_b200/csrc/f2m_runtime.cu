@@ -2406,7 +2406,9 @@ f2m_status f2m_solve_file(f2m_ctx* ctx, const char* path, int32_t top_k, const f
     }
     F2M_CUDA(cudaMemcpyAsync(&st, C.B.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (st != F2M_OK && st != kNeedsHost) return fail(ctx, (f2m_status)st, "the device solve stopped early");
+    // (kNeedsAxb: the host comb stage below solves the irregular combs)
+    if (st != F2M_OK && st != kNeedsHost && st != kNeedsAxb)
+        return fail(ctx, (f2m_status)st, "the device solve stopped early");
     if ((s = d2h(ctx, H.F, C.B.F, H.V)) || (s = d2h(ctx, H.efcnt, C.B.efcnt, H.V)) ||
         (s = d2h(ctx, H.ccnt, C.B.ccnt, H.V)) || (s = d2h(ctx, H.perm, C.B.perm, H.nbr.size())))
         return s;
