@@ -44,7 +44,7 @@ struct Batch {
     int32_t n_inst;
     int32_t N;              // neighbours selected per node (top_k, E_max)
     int32_t N_cut;          // top_k of the cut-off pass (FXY.hpp:77-78); normally N
-    int32_t skip_dedup;     // points were de-duplicated on the host already
+    int32_t skip_dedup;     // the points are distinct already
     int32_t cost_mode;      // f2m_cost_mode of the edge costs
     int32_t n_total;        // points over all instances (before de-duplication)
     const int64_t* offs;    // [n_inst+1]
@@ -209,6 +209,10 @@ double fp64_probe_ops(int kind, int blocks, int iters);
 cudaError_t launch_partition_check(int n_cases, unsigned long long seed, unsigned long long* bad,
                                    cudaStream_t s);
 cudaError_t launch_prep(const Batch& B, cudaStream_t s, int64_t* launches);
+// Rounding and de-duplication alone: fills dup_of and *count, the points that
+// repeat an earlier one.  Uses offs, X_in, Y_in, Pr, dup_of, the chunk lists and
+// 2 n_total ints at top_nbr.
+cudaError_t launch_find_repeats(const Batch& B, int32_t* count, cudaStream_t s, int64_t* launches);
 // Ax=b of the irregular combs and the primal of every instance the solver
 // left with status kNeedsAxb (one CTA per instance of the batch).
 cudaError_t launch_axb(const Batch& B, const DevParams& P, cudaStream_t s, int64_t* launches);

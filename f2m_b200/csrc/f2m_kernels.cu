@@ -109,6 +109,12 @@ __global__ void __launch_bounds__(kT) k_dup(Batch B) {
     const int j = DupTable(B, base, n).find(i, p.x, p.y);
     if (j != i) B.dup_of[base + i] = j;
 }
+// how many points repeat an earlier one
+__global__ void __launch_bounds__(kT) k_repeats(const int32_t* dup_of, int n, int32_t* count) {
+    const int i = blockIdx.x * kT + threadIdx.x;
+    const unsigned m = __ballot_sync(0xffffffffu, i < n && dup_of[i] >= 0);
+    if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, __popc(m));
+}
 
 /* ------------------------------------------------------------------ */
 /* k_prep: compaction, bbox, cell grid (FXY.hpp:231-309)                 */
@@ -1755,16 +1761,28 @@ cudaError_t launch_axb(const Batch& B, const DevParams& P, cudaStream_t s, int64
 /* ------------------------------------------------------------------ */
 /* host launchers                                                       */
 /* ------------------------------------------------------------------ */
-cudaError_t launch_prep(const Batch& B, cudaStream_t s, int64_t* launches) {
-    if (B.n_chunks > 0) {
-        if (!B.skip_dedup) {
-            cudaError_t e = cudaMemsetAsync(B.top_nbr, 0xff, sizeof(int32_t) * 2 * B.n_total, s);
-            if (e != cudaSuccess) return e;
-        }
-        k_round<<<B.n_chunks, kT, 0, s>>>(B);
-        if (!B.skip_dedup) k_dup<<<B.n_chunks, kT, 0, s>>>(B);
-        *launches += B.skip_dedup ? 1 : 2;
+static cudaError_t launch_round_dedup(const Batch& B, cudaStream_t s, int64_t* launches) {
+    if (B.n_chunks <= 0) return cudaSuccess;
+    if (!B.skip_dedup) {
+        cudaError_t e = cudaMemsetAsync(B.top_nbr, 0xff, sizeof(int32_t) * 2 * B.n_total, s);
+        if (e != cudaSuccess) return e;
     }
+    k_round<<<B.n_chunks, kT, 0, s>>>(B);
+    if (!B.skip_dedup) k_dup<<<B.n_chunks, kT, 0, s>>>(B);
+    *launches += B.skip_dedup ? 1 : 2;
+    return cudaGetLastError();
+}
+cudaError_t launch_find_repeats(const Batch& B, int32_t* count, cudaStream_t s, int64_t* launches) {
+    cudaError_t e = launch_round_dedup(B, s, launches);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(count, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
+    k_repeats<<<(unsigned)(((int64_t)B.n_total + kT - 1) / kT), kT, 0, s>>>(B.dup_of, B.n_total, count);
+    ++*launches;
+    return cudaGetLastError();
+}
+cudaError_t launch_prep(const Batch& B, cudaStream_t s, int64_t* launches) {
+    cudaError_t e = launch_round_dedup(B, s, launches);
+    if (e != cudaSuccess) return e;
     k_prep<<<B.n_inst, kT, 0, s>>>(B);
     ++*launches;
     return cudaGetLastError();

@@ -202,6 +202,24 @@ void make_plan(Plan& pl, int32_t n_inst, const int64_t* offs, int32_t N) {
     pl.S_cap = 2 * Neff * std::max<int64_t>(pl.n_total, 1);
 }
 
+// Work lists of one instance written on the device (no host staging).
+__global__ void k_single_lists(int64_t* offs, int32_t* chunk_inst, int32_t* chunk_start, int32_t* order,
+                                int32_t n, int32_t n_chunks) {
+    const int t = threadIdx.x;
+    if (t == 0) { offs[0] = 0; offs[1] = n; order[0] = 0; }
+    for (int c = t; c < n_chunks; c += blockDim.x) { chunk_inst[c] = 0; chunk_start[c] = c * kChunk; }
+}
+
+// A single instance whose distinct points are known: its class follows them.
+void replan_single(Plan& pl, int32_t V) {
+    pl.max_n = V;
+    pl.cnt.assign(pl.cnt.size(), 0);
+    pl.seg.assign(pl.seg.size(), 0);
+    const int c = solve_class_of(V, solve_wide_class(1));
+    pl.cnt[c] = 1;
+    pl.class_vcap[c] = std::max(V, 4);
+}
+
 // Carves every buffer of a batched call out of one arena.  With A.base ==
 // nullptr it only measures.
 void carve_grid(Arena& A, GridState& G, int64_t n, int64_t S) {
@@ -777,12 +795,15 @@ void carve_edge_sort(Arena& A, EdgeSort& E, int64_t S) {
 // 8,000 points 33.3 / 7.0.  Without coordinates (f2m_solve_graph) the CTAs' halos
 // are not local, so those keep the one SM.
 constexpr int32_t kGridSingle = 2500;
+bool takes_grid(int32_t n, int32_t n_inst, const f2m_params& prm, bool spatial) {
+    return n > solve_max_nodes() ||
+           (n_inst == 1 && (prm.solver == 2 || (prm.solver == 0 && spatial && n > kGridSingle)));
+}
 
 f2m_status setup_call(f2m_ctx* ctx, DevCall& C, int32_t n_inst, const int64_t* h_offs, int32_t top_k,
                       const f2m_params& prm, bool own_inputs, bool spatial = true) {
     make_plan(C.pl, n_inst, h_offs, top_k);
-    C.grid = C.pl.max_n > solve_max_nodes() ||
-             (n_inst == 1 && (prm.solver == 2 || (prm.solver == 0 && spatial && C.pl.max_n > kGridSingle)));
+    C.grid = takes_grid(C.pl.max_n, n_inst, prm, spatial);
     if (C.grid && n_inst > 1)
         return fail(ctx, F2M_ERR_CAPACITY, "batched instances are limited to " +
                                                std::to_string(solve_max_nodes()) +
@@ -843,6 +864,13 @@ f2m_status run_device(f2m_ctx* ctx, DevCall& C, const f2m_params& prm, bool buil
     Range rg("f2m enqueue device stages");
     F2M_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
     F2M_CUDA(launch_prep(C.B, ctx->stream, &ctx->launches));
+    if (C.grid) {  // one instance: its distinct points decide where it runs
+        int32_t V = 0;
+        F2M_CUDA(cudaMemcpyAsync(&V, C.B.Vn, sizeof(V), cudaMemcpyDeviceToHost, ctx->stream));
+        F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+        replan_single(C.pl, V);
+        C.grid = takes_grid(V, 1, prm, true);
+    }
     F2M_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
     F2M_CUDA(launch_knn(C.B, C.scan, ctx->stream, &ctx->launches));
     F2M_CUDA(cudaEventRecord(ctx->ev[2], ctx->stream));
@@ -1569,13 +1597,77 @@ f2m_status f2m_solve_batch_device(f2m_ctx* ctx, int32_t n_inst, const int64_t* h
 
 namespace {
 
+// The distinct points of a large instance, ahead of its plan: the solver, the
+// size class and the buffers (kilobytes a point) follow them, not the inputs.
+// The inputs stay where setup_call puts them (X, at the arena's start); the
+// kept points are compacted on the host when there are repeats.
+// (The graph alone has no solver to choose, so there the stage waits for sizes
+// whose buffers matter: its synchronisation costs 0.1 ms.)
+constexpr int32_t kRepeatStage = 16384;
+struct Distinct {
+    std::vector<double> x, y;  // empty: no repeats
+    std::vector<int32_t> label;
+    const double* X = nullptr;  // inputs on the device
+};
+f2m_status find_distinct(f2m_ctx* ctx, const double* x, const double* y, const int32_t* labels, int32_t n,
+                         Distinct& D) {
+    const int32_t nc = (n + kChunk - 1) / kChunk;
+    Batch B{};
+    int32_t *ci = nullptr, *cs = nullptr, *count = nullptr;
+    auto carve_in = [&](Arena& A) {
+        B.offs = A.take<int64_t>(2);
+        B.X_in = A.take<double>(n);
+        B.Y_in = A.take<double>(n);
+        B.Pr = A.take<double2>(n);
+        B.dup_of = A.take<int32_t>(n);
+        B.top_nbr = A.take<int32_t>(2 * (int64_t)n);
+        ci = A.take<int32_t>(nc);
+        cs = A.take<int32_t>(nc);
+        count = A.take<int32_t>(1);
+    };
+    Arena A;
+    carve_in(A);
+    F2M_CUDA(ensure_device(ctx, A.used));
+    A.base = ctx->dev;
+    A.used = 0;
+    carve_in(A);
+    B.n_inst = 1;
+    B.n_total = n;
+    B.chunk_inst = ci;
+    B.chunk_start = cs;
+    B.n_chunks = nc;
+    k_single_lists<<<1, 256, 0, ctx->stream>>>(const_cast<int64_t*>(B.offs), ci, cs, count, n, nc);
+    ctx->launches++;
+    F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(B.X_in), x, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(B.Y_in), y, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(launch_find_repeats(B, count, ctx->stream, &ctx->launches));
+    int32_t repeats = 0;
+    F2M_CUDA(cudaMemcpyAsync(&repeats, count, sizeof(repeats), cudaMemcpyDeviceToHost, ctx->stream));
+    F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    D.X = B.X_in;
+    if (repeats == 0) return F2M_OK;
+    std::vector<int32_t> dup(n);
+    F2M_CUDA(cudaMemcpyAsync(dup.data(), B.dup_of, n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    D.x.reserve(n - repeats);
+    D.y.reserve(n - repeats);
+    D.label.reserve(n - repeats);
+    for (int32_t i = 0; i < n; ++i) {
+        if (dup[i] >= 0) continue;
+        D.x.push_back(x[i]);
+        D.y.push_back(y[i]);
+        D.label.push_back(labels ? labels[i] : i + 1);
+    }
+    return F2M_OK;
+}
+
 // The single-instance path: rounding/de-duplication, kNN graph and, when
 // `solve`, the dual descent, comb stage and primal.
 f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int32_t* labels, int32_t n,
                        int32_t top_k, const f2m_params* params, bool solve, f2m_result** out,
                        const double* F0 = nullptr, int32_t nF0 = 0) {
     *out = nullptr;
-    const int64_t offs[2] = {0, n};
+    int64_t offs[2] = {0, n};
     f2m_status s = check_args(ctx, 1, offs, top_k, params);
     if (s) return s;
     f2m_params prm;
@@ -1584,8 +1676,23 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     cudaSetDevice(ctx->device);
     std::unique_ptr<f2m_result> R(new f2m_result());
     StageClock clk;
+    Distinct D;
+    const bool distinct = n > (solve ? kGridSingle : kRepeatStage);
+    if (distinct) {
+        if ((s = find_distinct(ctx, x, y, labels, n, D))) return s;
+        if (!D.x.empty()) {
+            x = D.x.data();
+            y = D.y.data();
+            labels = D.label.data();
+            n = (int32_t)D.x.size();
+            offs[1] = n;
+        }
+        clk.mark("distinct");
+    }
+    const size_t cap = ctx->dev_cap;
     DevCall C;
     if ((s = setup_call(ctx, C, 1, offs, top_k, prm, true))) return s;
+    C.B.skip_dedup = distinct ? 1 : 0;
     int32_t* dK = nullptr;
     if (labels) {
         // labels ride in the (unused) cursor buffer until k_prep compacts them
@@ -1594,8 +1701,10 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
         F2M_CUDA(cudaMemcpyAsync(dK, labels, n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     }
     F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(C.B.offs), offs, 2 * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-    F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.X_in), x, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.Y_in), y, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    if (!(distinct && D.x.empty() && ctx->dev_cap == cap && C.B.X_in == D.X)) {  // (else in place already)
+        F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.X_in), x, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+        F2M_CUDA(cudaMemcpyAsync(const_cast<double*>(C.B.Y_in), y, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    }
     auto t0 = std::chrono::steady_clock::now();
     F2M_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
     F2M_CUDA(launch_prep(C.B, ctx->stream, &ctx->launches));
@@ -2509,14 +2618,6 @@ cudaError_t noalloc_scratch(void** out) {
     return cudaSuccess;
 }
 
-// Work lists of one instance written on the device (no host staging).
-__global__ void k_noalloc_setup(int64_t* offs, int32_t* chunk_inst, int32_t* chunk_start, int32_t* order,
-                                int32_t n, int32_t n_chunks) {
-    const int t = threadIdx.x;
-    if (t == 0) { offs[0] = 0; offs[1] = n; order[0] = 0; }
-    for (int c = t; c < n_chunks; c += blockDim.x) { chunk_inst[c] = 0; chunk_start[c] = c * kChunk; }
-}
-
 // Copies the result out; an instance that needs the host comb stage is
 // reported as F2M_ERR_CAPACITY.
 __global__ void k_noalloc_finish(const int32_t* st_in, const double* lp_in, int32_t* st_out, double* lp_out) {
@@ -2565,7 +2666,7 @@ extern "C" f2m_status f2m_solve_points_noalloc(const double* d_x, const double* 
     B.Y_in = d_y;
     B.skip_dedup = 0;
     int64_t launches = 0;
-    k_noalloc_setup<<<1, 256, 0, s>>>(const_cast<int64_t*>(B.offs), ci, cs, ord, n, n_chunks);
+    k_single_lists<<<1, 256, 0, s>>>(const_cast<int64_t*>(B.offs), ci, cs, ord, n, n_chunks);
     if (cudaGetLastError() != cudaSuccess) return F2M_ERR_CUDA;
     if (launch_prep(B, s, &launches) != cudaSuccess || launch_knn(B, scan, s, &launches) != cudaSuccess ||
         launch_graph(B, deg, scan, s, &launches) != cudaSuccess ||
