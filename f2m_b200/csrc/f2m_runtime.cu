@@ -771,6 +771,7 @@ struct DevCall {
     GridState G{};
     bool grid = false;      // the single large instance runs on the grid-wide solver
     bool spatial = true;    // the grid solver's nodes can be ordered by their points (node = point)
+    bool ran_out = false;   // a barrier wait of a repair step on the grid-wide solver ran out
     int64_t* deg = nullptr;
     int64_t* scan = nullptr;
     int32_t *ci = nullptr, *cs = nullptr, *ord = nullptr;
@@ -798,6 +799,12 @@ constexpr int32_t kGridSingle = 2500;
 bool takes_grid(int32_t n, int32_t n_inst, const f2m_params& prm, bool spatial) {
     return n > solve_max_nodes() ||
            (n_inst == 1 && (prm.solver == 2 || (prm.solver == 0 && spatial && n > kGridSingle)));
+}
+
+// When a barrier wait of the whole-GPU solver runs out (grid_spin_limit), an
+// instance that was sent there for speed alone is solved again on one SM.
+bool retry_on_team(const DevCall& C, const f2m_params& prm) {
+    return C.grid && prm.solver == 0 && C.pl.max_n <= solve_max_nodes();
 }
 
 f2m_status setup_call(f2m_ctx* ctx, DevCall& C, int32_t n_inst, const int64_t* h_offs, int32_t top_k,
@@ -1039,6 +1046,11 @@ f2m_status complete_instance(f2m_ctx* ctx, DevCall& C, int b, const f2m_params& 
             int32_t st2 = 0;
             cudaMemcpyAsync(&st2, B.status + b, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream);
             if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) { ctx->err = cudaGetErrorString(e); return -1; }
+            if (st2 == F2M_ERR_CUDA) {  // its potentials are those of an abandoned solve
+                C.ran_out = true;
+                ctx->err = "a grid barrier wait ran out";
+                return -1;
+            }
             if (st2 == F2M_ERR_NOT_CONVERGED || st2 == F2M_ERR_CAPACITY) return -2;
             return HC.check();
         };
@@ -1541,7 +1553,13 @@ f2m_status f2m_solve_batch(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, co
     if (out->iterations) F2M_CUDA(cudaMemcpyAsync(out->iterations, C.B.iters, n_inst * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
     if (out->n_irregular) F2M_CUDA(cudaMemcpyAsync(out->n_irregular, C.B.n_irr, n_inst * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
-    if ((s = complete_batch(ctx, C, prm, status, lp, out->max_rank ? &mr : nullptr))) return s;
+    auto on_team = [&]() {  // (one instance)
+        prm.solver = 1;
+        return f2m_solve_batch(ctx, n_inst, offs, x, y, top_k, &prm, out);
+    };
+    if (status[0] == F2M_ERR_CUDA && retry_on_team(C, prm)) return on_team();
+    if ((s = complete_batch(ctx, C, prm, status, lp, out->max_rank ? &mr : nullptr)))
+        return C.ran_out && retry_on_team(C, prm) ? on_team() : s;
     std::memcpy(out->status, status.data(), n_inst * sizeof(int32_t));
     std::memcpy(out->lp, lp.data(), n_inst * sizeof(double));
     if (out->max_rank) std::memcpy(out->max_rank, mr.data(), n_inst * sizeof(int32_t));
@@ -1568,13 +1586,19 @@ f2m_status f2m_solve_batch_device(f2m_ctx* ctx, int32_t n_inst, const int64_t* h
     std::vector<int32_t> status(n_inst);
     F2M_CUDA(cudaMemcpyAsync(status.data(), C.B.status, n_inst * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    auto on_team = [&]() {  // (one instance)
+        prm.solver = 1;
+        return f2m_solve_batch_device(ctx, n_inst, h_offs, d_offs, d_x, d_y, top_k, &prm, d_out);
+    };
+    if (status[0] == F2M_ERR_CUDA && retry_on_team(C, prm)) return on_team();
     bool any = false;
     for (int32_t v : status) any |= (v == kNeedsHost);
     if (any) {
         std::vector<double> lp;
         if ((s = d2h(ctx, lp, C.B.lp, n_inst))) return s;
         F2M_CUDA(cudaStreamSynchronize(ctx->stream));
-        if ((s = complete_batch(ctx, C, prm, status, lp, nullptr))) return s;
+        if ((s = complete_batch(ctx, C, prm, status, lp, nullptr)))
+            return C.ran_out && retry_on_team(C, prm) ? on_team() : s;
         F2M_CUDA(cudaMemcpyAsync(C.B.lp, lp.data(), n_inst * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
         F2M_CUDA(cudaMemcpyAsync(C.B.status, status.data(), n_inst * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
         F2M_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1752,6 +1776,12 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     std::memcpy(&rp, ctx->pinned, sizeof(rp));
     const int32_t st = rp.status;
     clk.mark("device");
+    auto on_team = [&]() {
+        f2m_params q = prm;
+        q.solver = 1;
+        return points_call(ctx, x, y, labels, n, top_k, &q, solve, out, F0, nF0);
+    };
+    if (st == F2M_ERR_CUDA && retry_on_team(C, prm)) return on_team();
     if (st != F2M_OK && st != kNeedsHost) {
         R->status = st;
         R->err = st == F2M_ERR_INPUT ? "invalid instance (fewer than 4 distinct points or degenerate box)"
@@ -1772,7 +1802,7 @@ f2m_status points_call(f2m_ctx* ctx, const double* x, const double* y, const int
     } else {
         if ((s = pull_instance(ctx, C, 0, R->H, true))) return s;
         clk.mark("pull");
-        if ((s = complete_instance(ctx, C, 0, prm, *R))) return s;
+        if ((s = complete_instance(ctx, C, 0, prm, *R))) return C.ran_out && retry_on_team(C, prm) ? on_team() : s;
     }
     clk.mark("complete");
     if (st != F2M_OK && (s = pull_stats(ctx, C, 0, *R))) return s;
@@ -2515,6 +2545,11 @@ f2m_status f2m_solve_file(f2m_ctx* ctx, const char* path, int32_t top_k, const f
     }
     F2M_CUDA(cudaMemcpyAsync(&st, C.B.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    auto on_team = [&]() {
+        prm.solver = 1;
+        return f2m_solve_file(ctx, path, top_k, &prm, write_files, out);
+    };
+    if (st == F2M_ERR_CUDA && retry_on_team(C, prm)) return on_team();
     // (kNeedsAxb: the host comb stage below solves the irregular combs)
     if (st != F2M_OK && st != kNeedsHost && st != kNeedsAxb)
         return fail(ctx, (f2m_status)st, "the device solve stopped early");
@@ -2523,7 +2558,7 @@ f2m_status f2m_solve_file(f2m_ctx* ctx, const char* path, int32_t top_k, const f
         return s;
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
     if ((s = pull_stats(ctx, C, 0, *R))) return s;
-    if ((s = complete_instance(ctx, C, 0, prm, *R))) return s;
+    if ((s = complete_instance(ctx, C, 0, prm, *R))) return C.ran_out && retry_on_team(C, prm) ? on_team() : s;
     R->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if ((s = pull_stats(ctx, C, 0, *R))) return s;
     if (write_files) write_outputs(path, top_k, FP, dm, *R);

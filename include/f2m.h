@@ -58,14 +58,17 @@ typedef struct f2m_params {
     int64_t max_iters;     /* safety cap on Jacobi iterations per solve (not in the reference) */
     int32_t cost_mode;     /* f2m_cost_mode */
     int32_t solver;        /* 0 auto: a team per instance; a single instance above 2,500 points
-                              (10,000 from f2m_solve_graph) takes the whole GPU;
+                              (10,000 from f2m_solve_graph; distinct points count) takes the
+                              whole GPU;
                               1: a team up to 10,000 points (one SM: for callers that run many
                               single solves side by side, on a context per thread);
                               2: the whole-GPU solver for a single instance of any size */
     int64_t grid_spin_limit; /* the whole-GPU solver's grid barrier is a bounded wait: after
                               this many polls a CTA gives up, every CTA leaves the solve and
                               the call fails with F2M_ERR_CUDA (default 2^26, seconds of
-                              waiting; the GPU context stays usable).  Not in the reference. */
+                              waiting; the GPU context stays usable).  With solver 0 an
+                              instance that one SM can hold is then solved there instead.
+                              Not in the reference. */
 } f2m_params;
 
 typedef struct f2m_ctx f2m_ctx;
