@@ -16,6 +16,7 @@
 // chained through c_e = |p_a - p_b| to the coordinates.  All dual arithmetic
 // is FP64; coordinates and costs are FP32.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -185,39 +186,55 @@ __global__ void k_sfill(SmoothBatch S) {
     S.tnbr[S.tcap[gw] + S.N + p] = (int32_t)(g - S.offs[b]);
 }
 
-// sort each temporary list by neighbour, drop repeats and the -1 fillers
-__global__ void k_ssort(SmoothBatch S) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Sort each temporary list by neighbour, drop repeats and the -1 fillers, a warp
+// a list: up to 64 entries in registers, longer ones in place by the same
+// network with every comparison ascending (each merge starts with the mirrored
+// partner), where the missing entries up to a power of two would stay put.  (500
+// points, N = 48: 499 us with a thread a list in place, 627 through local memory,
+// 20 so.)
+__global__ void __launch_bounds__(128) k_ssort(SmoothBatch S) {
+    const int64_t g = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (g >= S.n_total) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned before = (1u << lane) - 1u;
     int32_t* a = S.tnbr + S.tcap[g];
     const int n = S.N + S.rdeg[g];
-    auto sort = [n](int32_t* out, const int32_t* in) {
-        for (int i = 0; i < n; ++i) {
-            const int32_t v = in[i];
-            int j = i - 1;
-            while (j >= 0 && out[j] > v) { out[j + 1] = out[j]; --j; }
-            out[j + 1] = v;
-        }
+    int m = 0, last = -1;  // entries kept, largest value so far
+    auto pack = [&](int32_t v) {  // 32 sorted values
+        int32_t prev = __shfl_up_sync(0xffffffffu, v, 1);
+        if (lane == 0) prev = last;
+        const bool keep = v != prev && v != INT_MAX;
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        if (keep) a[m + __popc(kept & before)] = v;
+        m += __popc(kept);
+        last = __shfl_sync(0xffffffffu, v, 31);
     };
-    int m = 0;
-    auto pack = [&](const int32_t* in) {
-        int32_t last = -1;
-        for (int i = 0; i < n; ++i) {
-            const int32_t v = in[i];
-            if (v > last) a[m++] = v;
-            last = max(last, v);
-        }
-    };
-    constexpr int kLocal = 96;  // lists up to this long are sorted in local memory
-    if (n <= kLocal) {
-        int32_t loc[kLocal];
-        sort(loc, a);
-        pack(loc);
+    if (n <= 64) {
+        int32_t v = lane < n ? a[lane] : INT_MAX, w = 32 + lane < n ? a[32 + lane] : INT_MAX;
+        __syncwarp();
+        warp_sort64(v, w);
+        pack(v);
+        pack(w);
     } else {
-        sort(a, a);
-        pack(a);
+        for (int k = 2; k < 2 * n; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int t = lane; t < n; t += 32) {
+                    const int u = j == k >> 1 ? t ^ (k - 1) : t ^ j;
+                    if (u <= t || u >= n) continue;
+                    const int32_t x = a[t], y = a[u];
+                    if (y < x) { a[t] = y; a[u] = x; }
+                }
+                __syncwarp();
+            }
+        }
+        for (int i = 0; i < n; i += 32) {
+            const int32_t v = i + lane < n ? a[i + lane] : INT_MAX;
+            __syncwarp();
+            pack(v);
+            __syncwarp();
+        }
     }
-    S.deg[g] = m;
+    if (lane == 0) S.deg[g] = m;
 }
 
 __global__ void k_scopy(SmoothBatch S) {
@@ -261,9 +278,14 @@ __global__ void k_smirror(SmoothBatch S) {
 // column with unit stride: from the rows its reads touched a sector a lane
 // (132 ms against 55 for the bound and gradient of 1,024 lattice instances).
 // With four lanes or more to a node, the per-step kernels, the rows are sectors.
+//
+// A warp a node sorts up to 64 entries in registers; the few longer lists rank
+// each entry among the others.  (500 points, N = 48: 170 us with a thread a list,
+// 8 so.)
 __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t g = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (g >= S.n_total) return;
+    const int lane = threadIdx.x & 31;
     const int64_t r0 = S.row[g];
     const int n = (int)(S.row[g + 1] - r0);
     auto key_of = [&](int k) { return ((unsigned long long)__float_as_uint(S.c[r0 + k]) << 32) | (unsigned)k; };
@@ -272,20 +294,14 @@ __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
         S.sent[r0 + k] = make_uint2((unsigned)(key >> 32), (unsigned)S.nbr[r0 + place]);
         S.splace[r0 + k] = place;
     };
-    constexpr int kLocal = 64;
-    if (n <= kLocal) {
-        unsigned long long loc[kLocal];
-        for (int k = 0; k < n; ++k) {
-            const unsigned long long x = key_of(k);
-            int j = k;
-            while (j > 0 && loc[j - 1] > x) { loc[j] = loc[j - 1]; --j; }
-            loc[j] = x;
-        }
-        for (int k = 0; k < n; ++k) put(k, loc[k]);
+    if (n <= 64) {
+        unsigned long long a = lane < n ? key_of(lane) : ~0ull, b = 32 + lane < n ? key_of(32 + lane) : ~0ull;
+        warp_sort64(a, b);
+        if (lane < n) put(lane, a);
+        if (32 + lane < n) put(32 + lane, b);
         return;
     }
-    // a long list (a hub): rank each entry among the others
-    for (int k = 0; k < n; ++k) {
+    for (int k = lane; k < n; k += 32) {
         const unsigned long long x = key_of(k);
         int rank = 0;
         for (int j = 0; j < n; ++j) rank += key_of(j) < x;
@@ -1025,12 +1041,12 @@ cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStrea
     *launches += 3;
     if ((e = launch_scan(S.deg, S.tcap, S.n_total, scan_scratch, s, launches)) != cudaSuccess) return e;
     k_sfill<<<nblk(nN, 256), 256, 0, s>>>(S);
-    k_ssort<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    k_ssort<<<nblk(S.n_total, 4), 128, 0, s>>>(S);
     *launches += 2;
     if ((e = launch_scan(S.deg, S.row, S.n_total, scan_scratch, s, launches)) != cudaSuccess) return e;
     k_scopy<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
     k_smirror<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
-    k_ssorted<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    k_ssorted<<<nblk(S.n_total, 4), 128, 0, s>>>(S);
     *launches += 3;
     if (S.W) {
         k_ssell<kCG><<<nblk(S.n_warps, 4), 128, 0, s>>>(S);
