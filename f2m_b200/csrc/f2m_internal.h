@@ -235,6 +235,17 @@ int solve_set_bounds(const int32_t* max_n);  // 3 increasing bounds; -1 if rejec
 void solve_get_bounds(int32_t* max_n);
 int solve_set_smem_kb(int kb);                // shared-memory target of a solver CTA (0 = all)
 int solve_get_smem_kb();
+// Entries further than this many tau past a node's third smallest are out of
+// reach of its root (f2m_smooth.cu says why they may be left out).
+constexpr double kReach = 50.0;
+constexpr int kReachCounters = 256;
+// What the graph build counts of the lists: entries within reach at u = 0, a node
+// on average, and the share of nodes with more than four lanes of the per-step
+// kernels hold.
+struct SmoothReach {
+    double mean = 0, over = 0;
+};
+constexpr int kStepScratch = 12;  // entries within reach that a lane keeps in shared memory
 // Smoothed-bound batch (f2m_smooth.cu).  Node g of instance b is offs[b] +
 // local id; neighbour ids in nbr are local; slots are global (row).
 struct SmoothBatch {
@@ -260,6 +271,8 @@ struct SmoothBatch {
     int64_t s_cap = 0;                  // entries of the [S] arrays
     uint2* sent = nullptr;              // [S] each list by ascending cost: cost bits, local neighbour
     int32_t* splace = nullptr;          // [S] place of that entry in the CSR row
+    unsigned long long* reach = nullptr;  // [2 kReachCounters] sums of SmoothReach over the nodes (or null)
+    int32_t lanes = 1;                  // lanes of a node (per-step path)
     double* gs = nullptr;               // [S] the steps' share of dL/dc, in that order
     uint2* sell = nullptr;              // [n_warps * 32 * W] the first entries of each list in slices of 32 lanes
     double* gsell = nullptr;            // [n_warps * 32 * W] their share of dL/dc
@@ -288,11 +301,16 @@ struct SmoothBatch {
 };
 cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStream_t s,
                                 int64_t* launches);
+cudaError_t launch_smooth_slices(SmoothBatch& S, cudaStream_t s, int64_t* launches);
 cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaStream_t s,
                                 int64_t* launches);
 cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches);
 int32_t smooth_max_nodes();
-int smooth_nodes_per_warp(bool steps, int64_t n_total);
+// Which path a call takes and its lanes a node; reach matters where
+// smooth_needs_reach says so.
+bool smooth_needs_reach(int32_t solver, int32_t n_inst, int64_t n_total, int sms);
+bool smooth_takes_steps(int32_t solver, int32_t n_inst, int sms, const SmoothReach& reach);
+int smooth_step_lanes(int64_t n_total, const SmoothReach& reach);
 // Rate probe of the smoothed bound's logistic term (one exp and one division,
 // the Newton sums' unit of work), and its work per launch.
 cudaError_t launch_logit_probe(int blocks, int iters, double* out, cudaStream_t s);

@@ -406,12 +406,12 @@ void parallel_for(int64_t n, Fn fn, int64_t serial_below = 20000) {
 // std::sort of a large array as sorted chunks merged pairwise, each level's
 // merges side by side (the keys here are unique, so the order is the same)
 template <class T, class Less>
-void parallel_sort(std::vector<T>& a, Less less, int64_t serial_below = 200000) {
+void parallel_sort(std::vector<T>& a, Less less) {
     const int64_t n = (int64_t)a.size();
     const int64_t hw = std::max(1u, std::thread::hardware_concurrency());
     int64_t parts = 1;
     while (parts * 2 <= std::min<int64_t>(hw, 32)) parts *= 2;
-    if (n < serial_below || parts < 2) { std::sort(a.begin(), a.end(), less); return; }
+    if (n < 200000 || parts < 2) { std::sort(a.begin(), a.end(), less); return; }
     std::vector<int64_t> b(parts + 1);
     for (int64_t p = 0; p <= parts; ++p) b[p] = n * p / parts;
     {
@@ -2000,7 +2000,7 @@ cudaError_t smooth_steps_graph(f2m_ctx* ctx, SmoothBatch& B, bool grad) {
     int64_t tb, ob;
     std::memcpy(&tb, &B.tau, 8);
     std::memcpy(&ob, &B.omega, 8);
-    const std::vector<int64_t> key{B.n_total, B.n_inst, B.n_warps, B.N, B.iters, B.ckpt, B.newton_max, grad ? 1 : 0,
+    const std::vector<int64_t> key{B.n_total, B.n_inst, B.n_warps, B.lanes, B.N, B.iters, B.ckpt, B.newton_max, grad ? 1 : 0,
                                    tb, ob, (int64_t)(intptr_t)ctx->dev, (int64_t)ctx->dev_cap};
     if (ctx->sgraph && key == ctx->skey) {
         ctx->launches += ctx->sgraph_launches;
@@ -2071,41 +2071,31 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     const int32_t K = sp.checkpoint;
     const int32_t nck = std::max(1, (sp.iters + K - 1) / K);
     const int64_t S = 2 * n * N + 8 * n;  // union lists: own N + reverse (+ slack)
-    // Under two instances an SM a pass of one CTA waits on its own latency and
-    // the whole GPU takes each pass instead.  So it does where tau is large
-    // against the point spacing (of the largest instance): whole lists are then
-    // within reach of a root (50 tau), more than a lane's scratch holds, and the
-    // lanes of a group share them.  Bound and gradient, 40 steps, one CTA each / a
-    // launch a pass, unit spacing: 600 instances of 100-500 points (N = 12) 7.0 /
-    // 9.0 ms at tau 1e-2, 18 / 9.9 at 5e-2; 600 of 200-1,500 (N = 28) 20.6 / 32.1
-    // and 65 / 44.
-    bool steps = sp.solver == 2;
-    if (sp.solver == 0) {
-        int32_t big = 0;
-        for (int32_t b = 1; b < n_inst; ++b)
-            if (offs[b + 1] - offs[b] > offs[big + 1] - offs[big]) big = b;
-        const auto bx = std::minmax_element(x + offs[big], x + offs[big + 1]);
-        const auto by = std::minmax_element(y + offs[big], y + offs[big + 1]);
-        const double w = (double)*bx.second - *bx.first, h = (double)*by.second - *by.first;
-        const double spacing = std::sqrt(w * h / (double)(offs[big + 1] - offs[big]));
-        steps = n_inst < 2 * ctx->sms || 50 * sp.tau > spacing;
-    }
-    std::vector<int64_t> sbase(n_inst + 1, 0);  // slices, or warps of the per-step kernels
-    const int64_t npw = smooth_nodes_per_warp(steps, n);
-    std::vector<int32_t> order(n_inst);
-    for (int32_t b = 0; b < n_inst; ++b) {
-        sbase[b + 1] = sbase[b] + (offs[b + 1] - offs[b] + npw - 1) / npw;
-        order[b] = b;
-    }
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t a, int32_t b) { return offs[a + 1] - offs[a] > offs[b + 1] - offs[b]; });
-    const int64_t n_warps = sbase[n_inst];
-    // slices hold 2 N entries of a node, nearly every list
-    const int32_t W = steps ? 0 : (int32_t)((2 * (int64_t)N * npw + 31) / 32);
+    // The path and its lanes a node follow, where they matter, how many list entries
+    // are within reach of a root, which the graph build counts.
+    const bool ask = smooth_needs_reach(sp.solver, n_inst, n, ctx->sms);
+    struct Path {
+        bool steps;
+        int lanes;
+        std::vector<int64_t> sbase;  // first slice, or warp of the per-step kernels, of each instance
+        int64_t n_warps;
+        int32_t W;                   // columns of a slice: 2 N entries of a node, nearly every list
+    };
+    auto path_of = [&](const SmoothReach& reach) {
+        Path q;
+        q.steps = smooth_takes_steps(sp.solver, n_inst, ctx->sms, reach);
+        q.lanes = q.steps ? smooth_step_lanes(n, reach) : 1;
+        const int64_t npw = 32 / q.lanes;
+        q.sbase.assign(n_inst + 1, 0);
+        for (int32_t b = 0; b < n_inst; ++b) q.sbase[b + 1] = q.sbase[b] + (offs[b + 1] - offs[b] + npw - 1) / npw;
+        q.n_warps = q.sbase[n_inst];
+        q.W = q.steps ? 0 : 2 * N;
+        return q;
+    };
     SmoothBatch B;
     int64_t* scan = nullptr;
     double* dLd = nullptr;
-    auto carve_s = [&](Arena& A) {
+    auto carve_graph = [&](Arena& A) {
         B.offs = A.take<int64_t>(n_inst + 1);
         B.x = A.take<float>(n);
         B.y = A.take<float>(n);
@@ -2120,16 +2110,19 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
         B.nbr = A.take<int32_t>(S);
         B.mirror = A.take<int64_t>(S);
         B.c = A.take<float>(S);
-        B.sbase = A.take<int64_t>(n_inst + 1);
-        B.order = A.take<int32_t>(n_inst);
         B.sent = A.take<uint2>(S);
         B.splace = A.take<int32_t>(S);
-        if (!steps) B.sell = A.take<uint2>(n_warps * 32 * W);
+        B.reach = A.take<unsigned long long>(2 * kReachCounters);
+    };
+    auto carve_path = [&](Arena& A, const Path& q) {
+        B.sbase = A.take<int64_t>(n_inst + 1);
+        B.order = A.take<int32_t>(n_inst);
+        if (!q.steps) B.sell = A.take<uint2>(q.n_warps * 32 * q.W);
         B.L = A.take<double>(n_inst);
         dLd = A.take<double>(n_inst);
         B.queue = A.take<int32_t>(1);
         B.work = A.take<unsigned long long>(1);
-        if (steps) {
+        if (q.steps) {
             B.ua = A.take<double>(n);
             B.ub = A.take<double>(n);
             B.Lp = A.take<double>(n);
@@ -2145,24 +2138,31 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
             B.segt = A.take<double>(n * K);
             B.segm = A.take<double>((int64_t)n_inst * K);
             B.gs = A.take<double>(S);
-            if (!steps) B.gsell = A.take<double>(n_warps * 32 * W);
+            if (!q.steps) B.gsell = A.take<double>(q.n_warps * 32 * q.W);
             B.gc = A.take<double>(S);
             B.gx = A.take<float>(n);
             B.gy = A.take<float>(n);
         }
     };
+    // buffers for whichever path the graph decides (the lanes do not change them)
     Arena A;
-    carve_s(A);
-    F2M_CUDA(ensure_device(ctx, A.used));
+    carve_graph(A);
+    const size_t graph_bytes = A.used;
+    size_t bytes = 0;
+    for (const double mean : {0.0, (double)INFINITY}) {
+        A.used = graph_bytes;
+        carve_path(A, path_of(SmoothReach{mean, 0.0}));
+        bytes = std::max(bytes, A.used);
+    }
+    F2M_CUDA(ensure_device(ctx, bytes));
     A.base = ctx->dev;
     A.used = 0;
-    carve_s(A);
+    carve_graph(A);
+    if (!ask) B.reach = nullptr;
     ctx->timed = false;  // the arena no longer holds a solve batch
     B.n_inst = n_inst;
     B.N = N;
     B.n_total = n;
-    B.W = W;
-    B.n_warps = n_warps;
     B.s_cap = S;
     B.tau = sp.tau;
     B.inv_tau = 1.0 / sp.tau;
@@ -2171,19 +2171,38 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     B.newton_max = sp.newton_max;
     B.ckpt = K;
     B.n_ck = nck;
-    B.dL = dLd;
-    std::vector<double> up(n_inst, 1.0);
-    if (dL) std::copy(dL, dL + n_inst, up.begin());
     F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(B.offs), offs, (n_inst + 1) * sizeof(int64_t),
                              cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<float*>(B.x), x, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<float*>(B.y), y, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    F2M_CUDA(launch_smooth_graph(B, scan, ctx->stream, &ctx->launches));
+    std::vector<int32_t> order(n_inst);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int32_t a, int32_t b) { return offs[a + 1] - offs[a] > offs[b + 1] - offs[b]; });
+    SmoothReach reach;
+    if (ask) {
+        unsigned long long counts[2 * kReachCounters], in = 0, over = 0;
+        F2M_CUDA(cudaMemcpyAsync(counts, B.reach, sizeof(counts), cudaMemcpyDeviceToHost, ctx->stream));
+        F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (int k = 0; k < kReachCounters; ++k) { in += counts[k]; over += counts[kReachCounters + k]; }
+        reach = SmoothReach{(double)in / (double)n, (double)over / (double)n};
+    }
+    const Path path = path_of(reach);
+    const bool steps = path.steps;
+    carve_path(A, path);
+    B.W = path.W;
+    B.n_warps = path.n_warps;
+    B.lanes = path.lanes;
+    B.dL = dLd;
+    std::vector<double> up(n_inst, 1.0);
+    if (dL) std::copy(dL, dL + n_inst, up.begin());
     F2M_CUDA(cudaMemcpyAsync(dLd, up.data(), n_inst * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(B.sbase), sbase.data(), (n_inst + 1) * sizeof(int64_t),
+    F2M_CUDA(cudaMemcpyAsync(const_cast<int64_t*>(B.sbase), path.sbase.data(), (n_inst + 1) * sizeof(int64_t),
                              cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(B.order), order.data(), n_inst * sizeof(int32_t),
                              cudaMemcpyHostToDevice, ctx->stream));
-    F2M_CUDA(launch_smooth_graph(B, scan, ctx->stream, &ctx->launches));
+    if (!steps) F2M_CUDA(launch_smooth_slices(B, ctx->stream, &ctx->launches));
     B.solver = steps ? 2 : 1;
     ctx->smooth_terms = -1;
     ctx->smooth_ms = 0.f;

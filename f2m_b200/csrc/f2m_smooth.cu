@@ -294,11 +294,26 @@ __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
         S.sent[r0 + k] = make_uint2((unsigned)(key >> 32), (unsigned)S.nbr[r0 + place]);
         S.splace[r0 + k] = place;
     };
+    // entries within reach of the first root (u = 0)
+    auto reach_of = [&](unsigned third) { return __uint_as_float(third) + (float)(kReach * S.tau); };
+    auto count = [&](int in) {
+        if (lane != 0) return;
+        unsigned long long* at = S.reach + blockIdx.x % kReachCounters;
+        atomicAdd(at, (unsigned long long)in);
+        if (in > 4 * kStepScratch) atomicAdd(at + kReachCounters, 1ull);
+    };
     if (n <= 64) {
         unsigned long long a = lane < n ? key_of(lane) : ~0ull, b = 32 + lane < n ? key_of(32 + lane) : ~0ull;
         warp_sort64(a, b);
         if (lane < n) put(lane, a);
         if (32 + lane < n) put(32 + lane, b);
+        if (S.reach) {
+            const float lim = reach_of(__shfl_sync(0xffffffffu, (unsigned)(a >> 32), 2));
+            auto in = [&](int k, unsigned long long key) {
+                return __ballot_sync(0xffffffffu, k < n && __uint_as_float((unsigned)(key >> 32)) <= lim);
+            };
+            count(__popc(in(lane, a)) + __popc(in(32 + lane, b)));
+        }
         return;
     }
     for (int k = lane; k < n; k += 32) {
@@ -306,6 +321,13 @@ __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
         int rank = 0;
         for (int j = 0; j < n; ++j) rank += key_of(j) < x;
         put(rank, x);
+    }
+    if (S.reach) {
+        __syncwarp();
+        const float lim = reach_of(S.sent[r0 + 2].x);
+        int in = 0;
+        for (int k = lane; k < n; k += 32) in += S.c[r0 + k] <= lim;
+        count(__reduce_add_sync(0xffffffffu, in));
     }
 }
 
@@ -380,8 +402,7 @@ __device__ __forceinline__ double root_step(const LogitAcc& r, double tau, doubl
 // at 1e-16.  They are left out; with tau at a hundredth of the point spacing
 // three to five of some thirty entries remain.  Since a_k >= c_k - max u, the
 // scan of the ascending costs ends at the first c_k above that bound.
-constexpr double kReach = 50.0;
-constexpr int kBuf = 12;  // entries within reach that a lane keeps in shared memory
+constexpr int kBuf = kStepScratch;
 
 // A group of G lanes holds a node, lane l its entries l, l + G, ...: the lanes'
 // reads of a column fill sectors, their exponentials run side by side, and sums
@@ -828,16 +849,8 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
 
 /* ---------------- one launch per step, all instances --------------------- */
 // G lanes per node, each instance's nodes from a whole warp on (sbase counts
-// warps); the potentials stay in global memory.  Few nodes leave SMs idle, so
-// more lanes share a node's exponentials; many nodes fill them, and the shuffles
-// of a wide group are wasted.  Bound and gradient (100 steps, N = 24) at G = 4 /
-// 8 / 16 / 32: 500 points 4.4 / 3.4 / 2.8 / 2.6 ms, 4,000 points 5.5 / 4.1 / 3.6
-// / 3.8, 10,000 points 6.0 / 5.5 / 5.9 / 7.0, 64 instances of 70,000 points in
-// all 8.7 / 10.9 / 16.0 / 22.0.
+// warps); the potentials stay in global memory.
 constexpr int kWT = 128;  // threads of a CTA
-static int steps_lanes(int64_t n_total) {
-    return n_total <= 3000 ? 32 : (n_total <= 7000 ? 16 : (n_total <= 14000 ? 8 : 4));
-}
 template <int kWG>
 struct SThread {
     RowPart<kWG> nd;
@@ -1035,6 +1048,7 @@ cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStrea
     cudaError_t e;
     const int64_t nN = S.n_total * S.N;
     if ((e = cudaMemsetAsync(S.rdeg, 0, sizeof(int32_t) * S.n_total, s)) != cudaSuccess) return e;
+    if (S.reach && (e = cudaMemsetAsync(S.reach, 0, sizeof(unsigned long long) * 2 * kReachCounters, s)) != cudaSuccess) return e;
     k_sknn<<<nblk(S.n_total, 8), 256, 0, s>>>(S);
     k_srdeg<<<nblk(nN, 256), 256, 0, s>>>(S);
     k_stcap<<<nblk(S.n_total, 256), 256, 0, s>>>(S);
@@ -1048,10 +1062,12 @@ cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStrea
     k_smirror<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
     k_ssorted<<<nblk(S.n_total, 4), 128, 0, s>>>(S);
     *launches += 3;
-    if (S.W) {
-        k_ssell<kCG><<<nblk(S.n_warps, 4), 128, 0, s>>>(S);
-        ++*launches;
-    }
+    return cudaGetLastError();
+}
+// The slices of the persistent kernel.
+cudaError_t launch_smooth_slices(SmoothBatch& S, cudaStream_t s, int64_t* launches) {
+    k_ssell<kCG><<<nblk(S.n_warps, 4), 128, 0, s>>>(S);
+    ++*launches;
     return cudaGetLastError();
 }
 // Zeroes the sums of the reverse steps.
@@ -1060,8 +1076,6 @@ static cudaError_t clear_smooth_sums(const SmoothBatch& S, cudaStream_t s) {
     if (e == cudaSuccess && S.W) e = cudaMemsetAsync(S.gsell, 0, sizeof(double) * S.n_warps * 32 * S.W, s);
     return e;
 }
-// nodes of a warp of the persistent kernel's slices, or of the per-step kernels
-int smooth_nodes_per_warp(bool steps, int64_t n_total) { return 32 / (steps ? steps_lanes(n_total) : kCG); }
 // dL/dc of every slot, then the coordinates
 static cudaError_t launch_smooth_coord(const SmoothBatch& S, cudaStream_t s, int64_t* launches) {
     k_s_merge<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
@@ -1123,8 +1137,43 @@ static cudaError_t launch_steps_of(SmoothBatch& S, bool grad, cudaStream_t s, in
     return launch_smooth_coord(S, s, launches);
 }
 
+// Under two instances an SM a pass of one CTA waits on its own latency, and the
+// whole GPU takes each pass instead.  So it does where more than nine list
+// entries are within reach of a root on average: a lane of the persistent kernel
+// holds a node alone, so its exponentials run one after the other and, past its
+// scratch, the list is gathered again for every Newton sum.  Bound and gradient,
+// 40 steps, 600 instances of 200-1,500 points, N = 24, persistent / per-step at
+// that average: lattice 12.6 / 23.4 ms at 3.4, 17.1 / 29.3 at 6.7, 35.0 / 33.5 at
+// 11.7, 58.1 / 37.8 at 25; uniform 23.9 / 32.4 at 6.6, 60.2 / 36.8 at 11.5;
+// clustered 30.0 / 33.8 at 6.1, 89.4 / 42.9 at 14.7.
+constexpr double kReachPersistent = 9.0;
+// Few nodes leave SMs idle, so more lanes share a node's exponentials; many nodes
+// fill them, and the shuffles of a wide group are wasted.  100 steps, N = 24, 4 /
+// 8 / 16 / 32 lanes: 500 points 4.4 / 3.4 / 2.8 / 2.6 ms, 4,000 points 5.5 / 4.1 /
+// 3.6 / 3.8, 10,000 points 6.0 / 5.5 / 5.9 / 7.0, 64 instances of 70,000 points in
+// all 8.7 / 10.9 / 16.0 / 22.0.  Four lanes hold 48 entries, and one list of a warp
+// past that makes the warp gather its lists again for every Newton sum: eight
+// lanes where that is common, at u = 0 or, from an average of about 30 on, as the
+// potentials move (40 steps, 4 / 8 lanes: 64 instances of 300-900 points, lattice
+// 4.1 / 4.6 ms at 25 entries, 5.4 / 5.1 at 31, clustered with 1% of the nodes past
+// 48 8.5 / 5.6 at 30; 600 of 200-1,500, uniform 55.6 / 59.8 at 31, lattice 102 / 77
+// at 35, clustered with 1% past 48 62.0 / 59.2 at 30, with 12% 103 / 70 at 39).
+constexpr int64_t kStepsMany = 14000, kStepsVeryMany = 150000;
+bool smooth_needs_reach(int32_t solver, int32_t n_inst, int64_t n_total, int sms) {
+    if (solver == 1) return false;
+    return (solver == 0 && n_inst >= 2 * sms) || n_total > kStepsMany;
+}
+bool smooth_takes_steps(int32_t solver, int32_t n_inst, int sms, const SmoothReach& reach) {
+    return solver == 2 || (solver == 0 && (n_inst < 2 * sms || reach.mean > kReachPersistent));
+}
+int smooth_step_lanes(int64_t n_total, const SmoothReach& reach) {
+    if (n_total > kStepsMany)
+        return reach.over > 0.005 || reach.mean > (n_total <= kStepsVeryMany ? 28 : 33) ? 8 : 4;
+    return n_total <= 3000 ? 32 : (n_total <= 7000 ? 16 : 8);
+}
+
 cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches) {
-    switch (steps_lanes(S.n_total)) {
+    switch (S.lanes) {
         case 4: return launch_steps_of<4>(S, grad, s, launches);
         case 8: return launch_steps_of<8>(S, grad, s, launches);
         case 16: return launch_steps_of<16>(S, grad, s, launches);
