@@ -254,28 +254,31 @@ struct SmoothBatch {
     const int64_t* offs = nullptr;
     const float* x = nullptr;
     const float* y = nullptr;
+    // graph build; the buffers of the bound and its adjoint follow on these
     unsigned long long* top = nullptr;  // [n_total * N] (cost bits << 32 | local index)
     int32_t* rdeg = nullptr;            // [n_total]
     int32_t* tcur = nullptr;            // [n_total]
     int64_t* tcap = nullptr;            // [n_total + 1] temporary list offsets
-    int32_t* tnbr = nullptr;            // [2 * n_total * N]
+    int32_t* tnbr = nullptr;            // [S] temporary lists (splace takes their place)
     int64_t* deg = nullptr;             // [n_total] scan input
     int64_t* row = nullptr;             // [n_total + 1]
     int32_t* nbr = nullptr;             // [S]
-    int64_t* mirror = nullptr;          // [S] slot of the same edge in the neighbour's list
     float* c = nullptr;                 // [S]
+    int32_t* splace = nullptr;          // [S] place in the CSR row of each entry by ascending cost
+    unsigned long long* reach = nullptr;  // [2 kReachCounters] sums of SmoothReach over the nodes (or null)
+    int64_t s_cap = 0;                  // S: entries of the [S] arrays
+    int32_t lanes = 1;                  // lanes of a node (per-step path)
     int32_t W = 0;                      // columns of a slice (0: per-step path, no slices)
-    int64_t n_warps = 0;                // slices, or warps of the per-step kernels (whole ones per instance)
+    int64_t n_warps = 0;                // warps of the per-step kernels (whole ones per instance) or, with
+                                        // slices, their places (whole sectors per instance)
     const int64_t* sbase = nullptr;     // [n_inst + 1] first of them of each instance
     const int32_t* order = nullptr;     // [n_inst] instances, largest first
-    int64_t s_cap = 0;                  // entries of the [S] arrays
     uint2* sent = nullptr;              // [S] each list by ascending cost: cost bits, local neighbour
-    int32_t* splace = nullptr;          // [S] place of that entry in the CSR row
-    unsigned long long* reach = nullptr;  // [2 kReachCounters] sums of SmoothReach over the nodes (or null)
-    int32_t lanes = 1;                  // lanes of a node (per-step path)
-    double* gs = nullptr;               // [S] the steps' share of dL/dc, in that order
-    uint2* sell = nullptr;              // [n_warps * 32 * W] the first entries of each list in slices of 32 lanes
-    double* gsell = nullptr;            // [n_warps * 32 * W] their share of dL/dc
+    uint2* sell = nullptr;              // [n_warps * W] the first entries of each list in slices of 32 nodes
+    // the steps' share of dL/dc, in that order, then (all of them added up) mirror:
+    double* gs = nullptr;               // [S]
+    double* gsell = nullptr;            // [n_warps * W]
+    int64_t* mirror = nullptr;          // [S] slot of the same edge in the neighbour's list
     double tau = 0, inv_tau = 0, omega = 0;
     int32_t iters = 0, newton_max = 0, ckpt = 1, n_ck = 1;
     double* L = nullptr;                // [n_inst]
@@ -301,7 +304,7 @@ struct SmoothBatch {
 };
 cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStream_t s,
                                 int64_t* launches);
-cudaError_t launch_smooth_slices(SmoothBatch& S, cudaStream_t s, int64_t* launches);
+cudaError_t launch_smooth_entries(SmoothBatch& S, cudaStream_t s, int64_t* launches);
 cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaStream_t s,
                                 int64_t* launches);
 cudaError_t launch_smooth_steps(SmoothBatch& S, bool grad, cudaStream_t s, int64_t* launches);

@@ -2068,17 +2068,25 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     const int64_t n = offs[n_inst];
     const bool grad = gx || gy;
     const int32_t N = top_k;
-    const int32_t K = sp.checkpoint;
-    const int32_t nck = std::max(1, (sp.iters + K - 1) / K);
-    const int64_t S = 2 * n * N + 8 * n;  // union lists: own N + reverse (+ slack)
+    // Steps of a segment that the adjoint recomputes at a time: as asked, but no more
+    // than there are, and the most whose iterates, roots and reach bounds take no
+    // more room than iterates and roots alone did with what else was kept a point.
+    // Results do not depend on it.
+    int32_t K = std::min(sp.checkpoint, std::max(sp.iters, 1));
+    auto checkpoints = [&](int64_t k) { return std::max<int64_t>(1, (sp.iters + k - 1) / k); };
+    const int64_t room = 16 * (int64_t)K + 8 * checkpoints(K) + 8 * (int64_t)N + 300;
+    for (int32_t k = K; k > 0; --k)
+        if (24 * (int64_t)k + 8 * checkpoints(k) <= room) { K = k; break; }
+    const int32_t nck = (int32_t)checkpoints(K);
+    const int64_t S = 2 * n * N;  // union lists: own N + reverse
     // The path and its lanes a node follow, where they matter, how many list entries
     // are within reach of a root, which the graph build counts.
     const bool ask = smooth_needs_reach(sp.solver, n_inst, n, ctx->sms);
     struct Path {
         bool steps;
         int lanes;
-        std::vector<int64_t> sbase;  // first slice, or warp of the per-step kernels, of each instance
-        int64_t n_warps;
+        std::vector<int64_t> sbase;  // places of the slices, or warps of the per-step kernels, before each instance
+        int64_t n_warps;             // all of them
         int32_t W;                   // columns of a slice: 2 N entries of a node, nearly every list
     };
     auto path_of = [&](const SmoothReach& reach) {
@@ -2087,7 +2095,10 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
         q.lanes = q.steps ? smooth_step_lanes(n, reach) : 1;
         const int64_t npw = 32 / q.lanes;
         q.sbase.assign(n_inst + 1, 0);
-        for (int32_t b = 0; b < n_inst; ++b) q.sbase[b + 1] = q.sbase[b] + (offs[b + 1] - offs[b] + npw - 1) / npw;
+        for (int32_t b = 0; b < n_inst; ++b) {
+            const int64_t v = offs[b + 1] - offs[b];
+            q.sbase[b + 1] = q.sbase[b] + (q.steps ? (v + npw - 1) / npw : (v + 3) & ~(int64_t)3);
+        }
         q.n_warps = q.sbase[n_inst];
         q.W = q.steps ? 0 : 2 * N;
         return q;
@@ -2099,25 +2110,25 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
         B.offs = A.take<int64_t>(n_inst + 1);
         B.x = A.take<float>(n);
         B.y = A.take<float>(n);
+        B.row = A.take<int64_t>(n + 1);
+        B.nbr = A.take<int32_t>(S);
+        B.c = A.take<float>(S);
+        B.tnbr = B.splace = A.take<int32_t>(S);
+        B.reach = A.take<unsigned long long>(2 * kReachCounters);
+    };
+    auto carve_build = [&](Arena& A) {
         B.top = A.take<unsigned long long>(n * N);
         B.rdeg = A.take<int32_t>(n);
         B.tcur = A.take<int32_t>(n);
         B.tcap = A.take<int64_t>(n + 1);
-        B.tnbr = A.take<int32_t>(S);
         B.deg = A.take<int64_t>(n);
-        B.row = A.take<int64_t>(n + 1);
         scan = A.take<int64_t>(scan_scratch_elems(n) + 1);
-        B.nbr = A.take<int32_t>(S);
-        B.mirror = A.take<int64_t>(S);
-        B.c = A.take<float>(S);
-        B.sent = A.take<uint2>(S);
-        B.splace = A.take<int32_t>(S);
-        B.reach = A.take<unsigned long long>(2 * kReachCounters);
     };
     auto carve_path = [&](Arena& A, const Path& q) {
         B.sbase = A.take<int64_t>(n_inst + 1);
         B.order = A.take<int32_t>(n_inst);
-        if (!q.steps) B.sell = A.take<uint2>(q.n_warps * 32 * q.W);
+        if (q.steps) B.sent = A.take<uint2>(S);
+        else B.sell = A.take<uint2>(q.n_warps * q.W);
         B.L = A.take<double>(n_inst);
         dLd = A.take<double>(n_inst);
         B.queue = A.take<int32_t>(1);
@@ -2137,8 +2148,8 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
             B.mu = A.take<double>(n);
             B.segt = A.take<double>(n * K);
             B.segm = A.take<double>((int64_t)n_inst * K);
-            B.gs = A.take<double>(S);
-            if (!q.steps) B.gsell = A.take<double>(q.n_warps * 32 * q.W);
+            B.gs = B.gsell = A.take<double>(std::max<int64_t>(S, q.n_warps * q.W));
+            B.mirror = reinterpret_cast<int64_t*>(B.gs);
             B.gc = A.take<double>(S);
             B.gx = A.take<float>(n);
             B.gy = A.take<float>(n);
@@ -2147,8 +2158,9 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     // buffers for whichever path the graph decides (the lanes do not change them)
     Arena A;
     carve_graph(A);
-    const size_t graph_bytes = A.used;
-    size_t bytes = 0;
+    const size_t graph_bytes = A.used;  // what only the build uses gives way to the path's buffers
+    carve_build(A);
+    size_t bytes = A.used;
     for (const double mean : {0.0, (double)INFINITY}) {
         A.used = graph_bytes;
         carve_path(A, path_of(SmoothReach{mean, 0.0}));
@@ -2158,6 +2170,8 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     A.base = ctx->dev;
     A.used = 0;
     carve_graph(A);
+    carve_build(A);
+    A.used = graph_bytes;
     if (!ask) B.reach = nullptr;
     ctx->timed = false;  // the arena no longer holds a solve batch
     B.n_inst = n_inst;
@@ -2202,7 +2216,7 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
                              cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(B.order), order.data(), n_inst * sizeof(int32_t),
                              cudaMemcpyHostToDevice, ctx->stream));
-    if (!steps) F2M_CUDA(launch_smooth_slices(B, ctx->stream, &ctx->launches));
+    F2M_CUDA(launch_smooth_entries(B, ctx->stream, &ctx->launches));
     B.solver = steps ? 2 : 1;
     ctx->smooth_terms = -1;
     ctx->smooth_ms = 0.f;

@@ -271,13 +271,14 @@ __global__ void k_smirror(SmoothBatch S) {
 
 /* ---------------- lists by ascending cost -------------------------------- */
 // A node root reads its list in ascending cost and stops early, so each list
-// is stored a second time sorted by (cost, neighbour): sent holds the cost bits
-// and the local neighbour, splace the entry's place in the CSR row.  The
-// persistent kernel, a lane or two to a node, reads the first entries from
-// slices of 32 lanes (ssell: column j of lane l at 32 j + l, S.W columns), a
-// column with unit stride: from the rows its reads touched a sector a lane
-// (132 ms against 55 for the bound and gradient of 1,024 lattice instances).
-// With four lanes or more to a node, the per-step kernels, the rows are sectors.
+// is stored a second time sorted by (cost, neighbour): splace holds each entry's
+// place in the CSR row, the entries are the cost bits and the local neighbour.
+// The persistent kernel, a lane to a node, reads the first S.W of them from slices
+// of 32 nodes (sell), a column with unit stride: from the rows its reads touched
+// a sector a lane (132 ms against 55 for the bound and gradient of 1,024 lattice
+// instances).  An instance's last slice is as wide as its nodes, rounded up to
+// whole sectors (sbase counts such places).  With four lanes or more to a node,
+// the per-step kernels, the rows (sent) are sectors.
 //
 // A warp a node sorts up to 64 entries in registers; the few longer lists rank
 // each entry among the others.  (500 points, N = 48: 170 us with a thread a list,
@@ -289,11 +290,7 @@ __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
     const int64_t r0 = S.row[g];
     const int n = (int)(S.row[g + 1] - r0);
     auto key_of = [&](int k) { return ((unsigned long long)__float_as_uint(S.c[r0 + k]) << 32) | (unsigned)k; };
-    auto put = [&](int k, unsigned long long key) {
-        const int place = (int)(unsigned)key;
-        S.sent[r0 + k] = make_uint2((unsigned)(key >> 32), (unsigned)S.nbr[r0 + place]);
-        S.splace[r0 + k] = place;
-    };
+    auto put = [&](int k, unsigned long long key) { S.splace[r0 + k] = (int)(unsigned)key; };
     // entries within reach of the first root (u = 0)
     auto reach_of = [&](unsigned third) { return __uint_as_float(third) + (float)(kReach * S.tau); };
     auto count = [&](int in) {
@@ -324,28 +321,42 @@ __global__ void __launch_bounds__(128) k_ssorted(SmoothBatch S) {
     }
     if (S.reach) {
         __syncwarp();
-        const float lim = reach_of(S.sent[r0 + 2].x);
+        const float lim = reach_of(__float_as_uint(S.c[r0 + S.splace[r0 + 2]]));
         int in = 0;
         for (int k = lane; k < n; k += 32) in += S.c[r0 + k] <= lim;
         count(__reduce_add_sync(0xffffffffu, in));
     }
 }
 
-template <int G>
+// entry j of the list at r0 in ascending cost
+__device__ __forceinline__ uint2 sorted_entry(const SmoothBatch& S, int64_t r0, int j) {
+    const int64_t k = r0 + S.splace[r0 + j];
+    return make_uint2(__float_as_uint(S.c[k]), (unsigned)S.nbr[k]);
+}
+// Where node v of an instance of V nodes, at place `base` of sbase, has its column
+// of a slice, and the distance between its entries.
+__device__ __forceinline__ int64_t slice_column(const SmoothBatch& S, int64_t base, int V, int v, int& stride) {
+    const int s0 = v & ~31;
+    stride = min(32, (V - s0 + 3) & ~3);
+    return (base + s0) * S.W + (v - s0);
+}
 __global__ void __launch_bounds__(128) k_ssell(SmoothBatch S) {
-    const int64_t w = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (w >= S.n_warps) return;
-    const int lane = threadIdx.x & 31;
-    const int b = find_inst(S.sbase, S.n_inst, w);
-    const int64_t g = S.offs[b] + (w - S.sbase[b]) * (32 / G) + lane / G;
-    const bool in = g < S.offs[b + 1];
-    const int64_t r0 = in ? S.row[g] : 0;
-    const int n = in ? (int)(S.row[g + 1] - r0) : 0;
-    uint2* out = S.sell + w * 32 * S.W + lane;
-    for (int j = 0; j < S.W; ++j) {
-        const int k = j * G + lane % G;
-        out[32 * j] = k < n ? S.sent[r0 + k] : make_uint2(0x7f800000u, 0u);
-    }
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= S.n_total) return;
+    const int b = find_inst(S.offs, S.n_inst, g);
+    int stride;
+    uint2* out = S.sell + slice_column(S, S.sbase[b], (int)(S.offs[b + 1] - S.offs[b]), (int)(g - S.offs[b]), stride);
+    const int64_t r0 = S.row[g];
+    const int n = min(S.W, (int)(S.row[g + 1] - r0));
+    for (int j = 0; j < n; ++j) out[(int64_t)stride * j] = sorted_entry(S, r0, j);
+}
+// the rows of the per-step kernels
+__global__ void __launch_bounds__(128) k_ssent(SmoothBatch S) {
+    const int64_t g = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (g >= S.n_total) return;
+    const int64_t r0 = S.row[g];
+    const int n = (int)(S.row[g + 1] - r0);
+    for (int j = threadIdx.x & 31; j < n; j += 32) S.sent[r0 + j] = sorted_entry(S, r0, j);
 }
 
 /* ---------------- node roots over the entries within reach --------------- */
@@ -418,14 +429,22 @@ struct RowPart {
     __device__ __forceinline__ uint2 get(int j) const { return ent[j * G]; }
     __device__ __forceinline__ double& acc(int j) const { return gs[j * G]; }
 };
-template <int G>
+struct SInst {
+    int b, V;
+    int64_t base, w0;    // first node, first place of its slices
+    const int64_t* row;  // row + base
+};
+// a node alone (G = 1): its column, and past W its CSR row
 struct SlicePart {
-    int n, deg, W;
-    const uint2* col;     // the lane's column of its slice
+    int n, deg, W, stride;
+    const uint2* col;
     double* gcol;
-    RowPart<G> row;       // the entries past W
-    __device__ __forceinline__ uint2 get(int j) const { return j < W ? col[32 * j] : row.get(j); }
-    __device__ __forceinline__ double& acc(int j) const { return j < W ? gcol[32 * j] : row.acc(j); }
+    const SmoothBatch* S;
+    int64_t r0;
+    __device__ __forceinline__ uint2 get(int j) const { return j < W ? col[stride * j] : sorted_entry(*S, r0, j); }
+    __device__ __forceinline__ double& acc(int j) const {
+        return j < W ? gcol[stride * j] : S->gc[r0 + S->splace[r0 + j]];
+    }
 };
 // of node v of the instance that starts at node `base` (no entries: in = false)
 template <int G>
@@ -441,16 +460,15 @@ __device__ __forceinline__ RowPart<G> row_part(const SmoothBatch& S, int64_t bas
     }
     return p;
 }
-template <int G>
-__device__ __forceinline__ SlicePart<G> slice_part(const SmoothBatch& S, int64_t base, int64_t w0, int v, bool in) {
-    SlicePart<G> p;
-    p.row = row_part<G>(S, base, v, in);
-    p.n = p.row.n;
-    p.deg = p.row.deg;
-    p.W = S.W;
-    const int64_t at = (w0 + v / (32 / G)) * 32 * S.W + (threadIdx.x & 31);
-    p.col = S.sell + at;
-    p.gcol = S.gsell + at;
+__device__ __forceinline__ SlicePart slice_part(const SmoothBatch& S, const SInst& I, int v, bool in) {
+    SlicePart p{0, 0, S.W, 0, nullptr, nullptr, &S, 0};
+    if (in) {
+        p.r0 = I.row[v];
+        p.n = p.deg = (int)(I.row[v + 1] - p.r0);
+        const int64_t at = slice_column(S, I.w0, I.V, v, p.stride);
+        p.col = S.sell + at;
+        p.gcol = S.gsell + at;
+    }
     return p;
 }
 template <int G>
@@ -660,12 +678,6 @@ __device__ __forceinline__ double node_rev2(const SmoothBatch& S, const List& L,
 }
 
 /* ---------------- the bound and its adjoint: one CTA per instance ------- */
-struct SInst {
-    int b, V;
-    int64_t base, w0;    // first node, first slice
-    const int64_t* row;  // row + base
-};
-constexpr int kCG = 1;  // lanes of a node
 
 // One damped Jacobi step u -> un; writes the roots and the reach bounds when
 // given, and the largest new potential into *umax_next.
@@ -673,12 +685,12 @@ __device__ __forceinline__ void sjacobi(const SmoothBatch& S, const SInst& I, co
                                         double* s_out, double* t_out, const SBuf& B, double umax,
                                         long long* umax_next, unsigned long long& terms) {
     double mx = -INFINITY;
-    const int v1 = (I.V + 32 / kCG - 1) / (32 / kCG) * (32 / kCG);  // whole warps
-    for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
-        const auto nd = slice_part<kCG>(S, I.base, I.w0, v, v < I.V);
+    const int v1 = (I.V + 31) & ~31;  // whole warps
+    for (int v = threadIdx.x; v < v1; v += kST) {
+        const auto nd = slice_part(S, I, v, v < I.V);
         double thr;
-        const double s = node_root<kCG>(S, nd, u, umax, B, &thr, terms);
-        if (v < I.V && threadIdx.x % kCG == 0) {
+        const double s = node_root<1>(S, nd, u, umax, B, &thr, terms);
+        if (v < I.V) {
             if (s_out) { s_out[v] = s; t_out[v] = thr; }
             const double x = (1.0 - S.omega) * u[v] + S.omega * s;
             un[v] = x;
@@ -738,7 +750,7 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
         I.V = (int)(S.offs[I.b + 1] - I.base);
         I.row = S.row + I.base;
         I.w0 = S.sbase[I.b];
-        const int v1 = (I.V + 32 / kCG - 1) / (32 / kCG) * (32 / kCG);
+        const int v1 = (I.V + 31) & ~31;
         double* Hb = Ha + max_v;
         const int T = S.iters, K = S.ckpt;
         double* ck = S.ck + I.base * S.n_ck;
@@ -822,22 +834,21 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
                 warp_ord_max(tm, &stmax[t & 1]);
                 __syncthreads();
                 const double umax = sm_[j], thrmax = ord_to(stmax[t & 1]);
-                const bool lead = threadIdx.x % kCG == 0;
-                for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
+                for (int v = threadIdx.x; v < v1; v += kST) {
                     const bool in = v < I.V;
-                    const auto nd = slice_part<kCG>(S, I.base, I.w0, v, in);
-                    const double m = node_rev1<kCG>(S, nd, (const double*)Ha, umax, B, in ? st[v] : 0.0,
+                    const auto nd = slice_part(S, I, v, in);
+                    const double m = node_rev1<1>(S, nd, (const double*)Ha, umax, B, in ? st[v] : 0.0,
                                                     in ? Hb[v] : 0.0, in ? lam[v] : 0.0, terms);
-                    if (in && lead) mu[v] = m;
+                    if (in) mu[v] = m;
                     __syncwarp();
                 }
                 __syncthreads();
-                for (int v = threadIdx.x / kCG; v < v1; v += kST / kCG) {
+                for (int v = threadIdx.x; v < v1; v += kST) {
                     const bool in = v < I.V;
-                    const auto nd = slice_part<kCG>(S, I.base, I.w0, v, in);
-                    const double x = node_rev2<kCG>(S, nd, in ? Ha[v] : 0.0, thrmax, (const double*)Hb, st,
+                    const auto nd = slice_part(S, I, v, in);
+                    const double x = node_rev2<1>(S, nd, in ? Ha[v] : 0.0, thrmax, (const double*)Hb, st,
                                                     (const double*)mu, B);
-                    if (in && lead) lam2[v] = (1.0 - S.omega) * lam[v] - x;
+                    if (in) lam2[v] = (1.0 - S.omega) * lam[v] - x;
                     __syncwarp();
                 }
                 __syncthreads();
@@ -1006,19 +1017,22 @@ __global__ void __launch_bounds__(kWT) k_sw_rev2(SmoothBatch S, const double* ut
     if (t.lead) lam2[t.g] = (1.0 - S.omega) * lam[t.g] - x;
 }
 
-// the steps' shares of dL/dc added to the slots
+// the steps' shares of dL/dc added to the slots (the persistent kernel adds those
+// past its slices itself)
 __global__ void __launch_bounds__(128) k_s_merge(SmoothBatch S) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= S.n_total) return;
-    const int64_t r0 = S.row[g], r1 = S.row[g + 1];
-    int64_t at = 0;
-    if (S.W) {
-        const int b = find_inst(S.offs, S.n_inst, g);
-        const int v = (int)(g - S.offs[b]);
-        at = (S.sbase[b] + v / (32 / kCG)) * 32 * S.W + (v % (32 / kCG)) * kCG;
+    const int64_t r0 = S.row[g];
+    const int n = (int)(S.row[g + 1] - r0);
+    if (!S.W) {
+        for (int k = 0; k < n; ++k) S.gc[r0 + S.splace[r0 + k]] += S.gs[r0 + k];
+        return;
     }
-    for (int k = 0; k < (int)(r1 - r0); ++k)
-        S.gc[r0 + S.splace[r0 + k]] += k / kCG < S.W ? S.gsell[at + 32 * (k / kCG) + k % kCG] : S.gs[r0 + k];
+    const int b = find_inst(S.offs, S.n_inst, g);
+    int stride;
+    const double* col =
+        S.gsell + slice_column(S, S.sbase[b], (int)(S.offs[b + 1] - S.offs[b]), (int)(g - S.offs[b]), stride);
+    for (int k = 0; k < min(n, S.W); ++k) S.gc[r0 + S.splace[r0 + k]] += col[(int64_t)stride * k];
 }
 
 __global__ void k_sw_coord(SmoothBatch S) {
@@ -1059,28 +1073,28 @@ cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStrea
     *launches += 2;
     if ((e = launch_scan(S.deg, S.row, S.n_total, scan_scratch, s, launches)) != cudaSuccess) return e;
     k_scopy<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
-    k_smirror<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
     k_ssorted<<<nblk(S.n_total, 4), 128, 0, s>>>(S);
     *launches += 3;
     return cudaGetLastError();
 }
-// The slices of the persistent kernel.
-cudaError_t launch_smooth_slices(SmoothBatch& S, cudaStream_t s, int64_t* launches) {
-    k_ssell<kCG><<<nblk(S.n_warps, 4), 128, 0, s>>>(S);
+// The sorted entries, in slices or rows as the path reads them.
+cudaError_t launch_smooth_entries(SmoothBatch& S, cudaStream_t s, int64_t* launches) {
+    if (S.W) k_ssell<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    else k_ssent<<<nblk(S.n_total, 4), 128, 0, s>>>(S);
     ++*launches;
     return cudaGetLastError();
 }
 // Zeroes the sums of the reverse steps.
 static cudaError_t clear_smooth_sums(const SmoothBatch& S, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(S.gs, 0, sizeof(double) * S.s_cap, s);
-    if (e == cudaSuccess && S.W) e = cudaMemsetAsync(S.gsell, 0, sizeof(double) * S.n_warps * 32 * S.W, s);
-    return e;
+    return S.W ? cudaMemsetAsync(S.gsell, 0, sizeof(double) * S.n_warps * S.W, s)
+               : cudaMemsetAsync(S.gs, 0, sizeof(double) * S.s_cap, s);
 }
 // dL/dc of every slot, then the coordinates
 static cudaError_t launch_smooth_coord(const SmoothBatch& S, cudaStream_t s, int64_t* launches) {
     k_s_merge<<<nblk(S.n_total, 128), 128, 0, s>>>(S);
+    k_smirror<<<nblk(S.n_total, 128), 128, 0, s>>>(S);  // (over the steps' shares, merged now)
     k_sw_coord<<<nblk(S.n_total, 256), 256, 0, s>>>(S);
-    *launches += 2;
+    *launches += 3;
     return cudaGetLastError();
 }
 
