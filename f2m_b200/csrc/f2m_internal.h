@@ -220,14 +220,17 @@ cudaError_t launch_knn(const Batch& B, int64_t* scan_scratch, cudaStream_t s, in
 cudaError_t launch_graph(const Batch& B, int64_t* deg_scratch, int64_t* scan_scratch,
                          cudaStream_t s, int64_t* launches);
 // Persistent solver over items[0..n_items) of size class c (largest first);
-// queue is a device counter.  REFIT variant: F += shift, frozen iterations,
-// run_fix (graph_cuda_comb.hpp:542-574).
+// queue is a device counter.
 cudaError_t launch_solve_class(int c, const Batch& B, const DevParams& P, const int32_t* items,
                                int n_items, int32_t* queue, int vcap, cudaStream_t s,
                                int64_t* launches);
-cudaError_t launch_refit_class(int c, const Batch& B, const DevParams& P, const int32_t* items,
-                               int n_items, int32_t* queue, int vcap, cudaStream_t s,
-                               int64_t* launches);
+// One instance on a team of the widest class, the class of every call of one;
+// and its repair step: F += shift, frozen iterations, run_fix
+// (graph_cuda_comb.hpp:542-574).
+cudaError_t launch_solve_one(const Batch& B, const DevParams& P, const int32_t* item, int32_t* queue,
+                             int vcap, cudaStream_t s, int64_t* launches);
+cudaError_t launch_refit_one(const Batch& B, const DevParams& P, const int32_t* item, int32_t* queue,
+                             int vcap, cudaStream_t s, int64_t* launches);
 int solve_num_classes();
 int solve_wide_class(int64_t n_inst);
 int solve_class_of(int32_t n, int wide);

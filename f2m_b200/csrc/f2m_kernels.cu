@@ -1971,28 +1971,24 @@ static cudaError_t launch_one(const Batch& B, const DevParams& P, const int32_t*
     return cudaGetLastError();
 }
 
-template <bool R>
-static cudaError_t launch_class(int c, const Batch& B, const DevParams& P, const int32_t* items,
-                                int n_items, int32_t* queue, int vcap, cudaStream_t s,
-                                int64_t* launches) {
-    if (n_items <= 0) return cudaSuccess;
-    switch (c) {
-        case 0: return launch_one<128, 8, R>(B, P, items, n_items, queue, vcap, s, launches);
-        case 1: return launch_one<256, 4, R>(B, P, items, n_items, queue, vcap, s, launches);
-        case 2: return launch_one<512, 2, R>(B, P, items, n_items, queue, vcap, s, launches);
-        default: return launch_one<1024, 1, R>(B, P, items, n_items, queue, vcap, s, launches);
-    }
-}
-
 cudaError_t launch_solve_class(int c, const Batch& B, const DevParams& P, const int32_t* items,
                                int n_items, int32_t* queue, int vcap, cudaStream_t s,
                                int64_t* launches) {
-    return launch_class<false>(c, B, P, items, n_items, queue, vcap, s, launches);
+    if (n_items <= 0) return cudaSuccess;
+    switch (c) {
+        case 0: return launch_one<128, 8, false>(B, P, items, n_items, queue, vcap, s, launches);
+        case 1: return launch_one<256, 4, false>(B, P, items, n_items, queue, vcap, s, launches);
+        case 2: return launch_one<512, 2, false>(B, P, items, n_items, queue, vcap, s, launches);
+        default: return launch_one<1024, 1, false>(B, P, items, n_items, queue, vcap, s, launches);
+    }
 }
-cudaError_t launch_refit_class(int c, const Batch& B, const DevParams& P, const int32_t* items,
-                               int n_items, int32_t* queue, int vcap, cudaStream_t s,
-                               int64_t* launches) {
-    return launch_class<true>(c, B, P, items, n_items, queue, vcap, s, launches);
+cudaError_t launch_solve_one(const Batch& B, const DevParams& P, const int32_t* item, int32_t* queue,
+                             int vcap, cudaStream_t s, int64_t* launches) {
+    return launch_one<1024, 1, false>(B, P, item, 1, queue, vcap, s, launches);
+}
+cudaError_t launch_refit_one(const Batch& B, const DevParams& P, const int32_t* item, int32_t* queue,
+                             int vcap, cudaStream_t s, int64_t* launches) {
+    return launch_one<1024, 1, true>(B, P, item, 1, queue, vcap, s, launches);
 }
 
 }  // namespace f2m

@@ -210,14 +210,11 @@ __global__ void k_single_lists(int64_t* offs, int32_t* chunk_inst, int32_t* chun
     for (int c = t; c < n_chunks; c += blockDim.x) { chunk_inst[c] = 0; chunk_start[c] = c * kChunk; }
 }
 
-// A single instance whose distinct points are known: its class follows them.
+// A single instance whose distinct points are known (the widest class, as every
+// call of one instance takes).
 void replan_single(Plan& pl, int32_t V) {
     pl.max_n = V;
-    pl.cnt.assign(pl.cnt.size(), 0);
-    pl.seg.assign(pl.seg.size(), 0);
-    const int c = solve_class_of(V, solve_wide_class(1));
-    pl.cnt[c] = 1;
-    pl.class_vcap[c] = std::max(V, 4);
+    pl.class_vcap.back() = std::max(V, 4);
 }
 
 // Carves every buffer of a batched call out of one arena.  With A.base ==
@@ -1034,8 +1031,8 @@ f2m_status complete_instance(f2m_ctx* ctx, DevCall& C, int b, const f2m_params& 
                 (e = cudaMemcpyAsync(C.ord, &one, sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(B.status + b, &st, sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
                 (e = (C.grid ? launch_solve_grid(B, to_dev(prm), C.G, b, H.V, true, ctx->stream, &ctx->launches)
-                             : launch_refit_class(solve_class_of(H.V, solve_wide_class(1)), B, to_dev(prm), C.ord, 1, B.queue + 7,
-                                                  std::max<int32_t>(H.V, 4), ctx->stream, &ctx->launches))) != cudaSuccess ||
+                             : launch_refit_one(B, to_dev(prm), C.ord, B.queue + 7, std::max<int32_t>(H.V, 4), ctx->stream,
+                                                &ctx->launches))) != cudaSuccess ||
                 (e = cudaMemcpyAsync(H.F.data(), B.F + ibase, H.V * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(H.efcnt.data(), B.efcnt + ibase, H.V * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(H.ccnt.data(), B.ccnt + ibase, H.V * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
@@ -2568,13 +2565,10 @@ f2m_status f2m_solve_file(f2m_ctx* ctx, const char* path, int32_t top_k, const f
         F2M_CUDA(launch_grid_order(C.B, C.G, 0, H.V, C.G.own, true, ctx->stream, &ctx->launches));
         F2M_CUDA(launch_solve_grid(C.B, to_dev(prm), C.G, 0, H.V, false, ctx->stream, &ctx->launches));
     } else {
-        // the host-assembled graph may have fewer nodes than points: re-plan
-        // the class from the node count
         std::vector<int32_t> one{0};
-        const int c = solve_class_of(H.V, solve_wide_class(1));
         F2M_CUDA(cudaMemcpyAsync(C.ord, one.data(), sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
-        F2M_CUDA(launch_solve_class(c, C.B, to_dev(prm), C.ord, 1, C.B.queue + 6,
-                                    std::max<int32_t>(H.V, 4), ctx->stream, &ctx->launches));
+        F2M_CUDA(launch_solve_one(C.B, to_dev(prm), C.ord, C.B.queue + 6, std::max<int32_t>(H.V, 4), ctx->stream,
+                                  &ctx->launches));
     }
     F2M_CUDA(cudaMemcpyAsync(&st, C.B.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -2738,8 +2732,7 @@ extern "C" f2m_status f2m_solve_points_noalloc(const double* d_x, const double* 
     if (cudaGetLastError() != cudaSuccess) return F2M_ERR_CUDA;
     if (launch_prep(B, s, &launches) != cudaSuccess || launch_knn(B, scan, s, &launches) != cudaSuccess ||
         launch_graph(B, deg, scan, s, &launches) != cudaSuccess ||
-        launch_solve_class(solve_class_of(n, solve_wide_class(1)), B, to_dev(prm), ord, 1, B.queue, std::max<int32_t>(n, 4), s,
-                           &launches) != cudaSuccess ||
+        launch_solve_one(B, to_dev(prm), ord, B.queue, std::max<int32_t>(n, 4), s, &launches) != cudaSuccess ||
         launch_axb(B, to_dev(prm), s, &launches) != cudaSuccess)
         return F2M_ERR_CUDA;
     k_noalloc_finish<<<1, 32, 0, s>>>(B.status, B.lp, d_status, d_lp);
