@@ -94,6 +94,7 @@ EXPORTS = [
     "f2m_get_class_bounds", "f2m_solve_graph", "f2m_solve_points_from", "f2m_fp64_rate",
     "f2m_partition_selfcheck", "f2m_smooth_work",
     "f2m_smoothed_bound_bwd_edges", "f2m_set_solver_smem_kb", "f2m_get_solver_smem_kb",
+    "f2m_batch_potentials", "f2m_team_width",
 ]
 
 _lib = None
@@ -135,6 +136,9 @@ def lib():
         L.f2m_result_nodes.argtypes = [vp] * 3
         L.f2m_result_stats.argtypes = [vp, P(Stats)]
         L.f2m_phase_times.argtypes = [vp, vp, P(Work)]
+        L.f2m_batch_potentials.argtypes = [vp, vp]
+        L.f2m_team_width.argtypes = [i32, i32]
+        L.f2m_team_width.restype = i32
         L.f2m_fp64_rate.argtypes = [vp, i32, i32, P(dbl)]
         L.f2m_partition_selfcheck.argtypes = [vp, i32, ctypes.c_uint64, P(ctypes.c_int64)]
         L.f2m_smooth_work.argtypes = [vp, P(ctypes.c_int64), P(ctypes.c_float)]
@@ -174,6 +178,11 @@ def get_class_bounds():
     b = np.zeros(3, np.int32)
     lib().f2m_get_class_bounds(b.ctypes.data_as(ctypes.c_void_p))
     return [int(v) for v in b]
+
+
+def team_width(n, n_inst):
+    """Threads of the team that solves an instance of n points in a call of n_inst."""
+    return lib().f2m_team_width(n, n_inst)
 
 
 def set_solver_smem_kb(kb):
@@ -297,6 +306,13 @@ class Context:
         w = Work()
         self._check(lib().f2m_phase_times(self._h, _ptr(ms), ctypes.byref(w)))
         return ms, {k: getattr(w, k) for k, _ in Work._fields_}
+
+    def batch_potentials(self, n_points):
+        """Potentials of the last batched solve (n_points: the points of that call),
+        instance b's from offs[b] on, before any other call on the context."""
+        F = np.zeros(n_points, np.float64)
+        self._check(lib().f2m_batch_potentials(self._h, _ptr(F)))
+        return F
 
     def fp64_rate(self, kind=0, repeats=3):
         """Measured FP64 pipe rate of this GPU, FP64 lane operations per second

@@ -234,6 +234,7 @@ cudaError_t launch_refit_one(const Batch& B, const DevParams& P, const int32_t* 
 int solve_num_classes();
 int solve_wide_class(int64_t n_inst);
 int solve_class_of(int32_t n, int wide);
+int solve_team_width(int c);
 int solve_set_bounds(const int32_t* max_n);  // 3 increasing bounds; -1 if rejected
 void solve_get_bounds(int32_t* max_n);
 int solve_set_smem_kb(int kb);                // shared-memory target of a solver CTA (0 = all)

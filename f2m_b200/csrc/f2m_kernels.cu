@@ -1862,6 +1862,7 @@ void solve_get_bounds(int32_t* max_n) {
 
 int32_t solve_max_nodes() { return 10000; }
 int solve_num_classes() { return kNumClasses; }
+int solve_team_width(int c) { return kClasses[c].team; }
 // The narrowest class for a call of n_inst instances: the widest one whose
 // teams are all resident at once.  The size bounds are for throughput, a full
 // GPU; a call with fewer instances than that leaves SMs idle, and a solve is

@@ -1321,6 +1321,14 @@ f2m_status f2m_phase_times(f2m_ctx* ctx, float* ms, f2m_work* work) {
     return F2M_OK;
 }
 
+f2m_status f2m_batch_potentials(f2m_ctx* ctx, double* F) {
+    if (!ctx || !F || !ctx->timed) return fail(ctx, F2M_ERR_INPUT, "no batched solve to read");
+    F2M_CUDA(cudaMemcpyAsync(F, ctx->last.F, ctx->last.n_total * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    F2M_CUDA(cudaStreamSynchronize(ctx->stream));
+    return F2M_OK;
+}
+int32_t f2m_team_width(int32_t n, int32_t n_inst) { return solve_team_width(solve_class_of(n, solve_wide_class(n_inst))); }
+
 const char* f2m_last_error(const f2m_ctx* c) { return c ? c->err.c_str() : "no context"; }
 int64_t f2m_kernel_launches(const f2m_ctx* c) { return c ? c->launches : 0; }
 

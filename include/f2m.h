@@ -140,6 +140,14 @@ typedef struct f2m_work {
  * reference counterpart (the reference prints gettimeofday phase times,
  * graph_cuda_define.hpp:29-34). */
 f2m_status f2m_phase_times(f2m_ctx* ctx, float* ms, f2m_work* work);
+/* Potentials of the last batched solve of this context: instance b's are at F +
+ * offs[b], one per distinct point in input order (n_nodes[b] of them; the rest of
+ * its range is not written).  F holds as many values as the call had points.
+ * Before any other call on the context. */
+f2m_status f2m_batch_potentials(f2m_ctx* ctx, double* F);
+/* Threads of the team that solves an instance of n points in a batched call of
+ * n_inst instances (see f2m_set_class_bounds). */
+int32_t f2m_team_width(int32_t n, int32_t n_inst);
 
 /* Measured FP64 pipe rate of this context's GPU in FP64 lane operations per
  * second (diagnostics; no reference counterpart).  The dual descent issues
@@ -337,10 +345,11 @@ int32_t f2m_smooth_max_nodes(void);
  * of at most max_nodes[0] points runs on a 128-thread team (8 per CTA), up to
  * max_nodes[1] on 256 (4 per CTA), up to max_nodes[2] on 512 (2 per CTA),
  * larger ones on 1024 threads.  A call with too few instances to fill the GPU
- * with teams of that width takes wider ones.  The potentials do not depend on the classes
- * (the LP value only through the order of its team-wide sum, ~1e-16
- * relative); f2m_b200/autotune.py times candidate bounds on a workload.  The
- * bounds are process-wide: set them before solving.  F2M_ERR_INPUT if not
+ * with teams of that width takes wider ones.  The potentials do not depend on
+ * the team, the LP value only through the order of its team-wide sum (~1e-16
+ * relative).  f2m_b200/autotune.py times candidate bounds
+ * on a workload.  The bounds are process-wide: set them before solving.
+ * F2M_ERR_INPUT if not
  * increasing or a class's shared memory cannot hold an instance that size. */
 f2m_status f2m_set_class_bounds(const int32_t* max_nodes); /* 3 values */
 void f2m_get_class_bounds(int32_t* max_nodes);
