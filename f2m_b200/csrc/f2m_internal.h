@@ -36,6 +36,7 @@ struct DevParams {
     int32_t ef_small_deg, ef_min;
     int64_t max_iters;
     int64_t spin_limit;     // grid barrier polls before giving up (whole-GPU solver)
+    int32_t class_max_n[3]; // size bounds of the three narrower team classes
 };
 
 // Pointers of one batched call.  Node g of instance b lives at index

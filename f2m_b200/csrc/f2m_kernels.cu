@@ -1588,8 +1588,14 @@ struct Solver {
             }
         // primal (graph_cuda.cu:135-147): x = 1 on A edges, 1/2 on the B edges
         // of regular combs; OVAL = sum x*Do, MAX edge rank (graph_tour.hpp:165-184)
+        // The sums take the order of the team that the instance's size asks for (threads
+        // past it add zeros), so that their bits do not depend on how many instances
+        // share the call.
+        const int n_in = (int)(B.offs[b + 1] - B.offs[b]);
+        const int team = min(TEAM, n_in <= P.class_max_n[0] ? 128 : n_in <= P.class_max_n[1] ? 256
+                                   : n_in <= P.class_max_n[2] ? 512 : 1024);
         PrimalSums ps;
-        for (int v = T.tid; v < V; v += TEAM)
+        for (int v = T.tid < team ? T.tid : V; v < V; v += team)
             primal_node(B, I, Hc, (const int*)nullptr, (const int*)nullptr, false, v, porog, ps);
         double lp = ps.lp, dual_neg = ps.dual_neg, fsum = ps.fsum;
         long long maxr = ps.maxr, viol = ps.viol;

@@ -143,6 +143,7 @@ DevParams to_dev(const f2m_params& p) {
     d.ef_min = p.ef_min;
     d.max_iters = p.max_iters;
     d.spin_limit = p.grid_spin_limit > 0 ? p.grid_spin_limit : 1;
+    solve_get_bounds(d.class_max_n);
     return d;
 }
 

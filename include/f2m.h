@@ -346,11 +346,12 @@ int32_t f2m_smooth_max_nodes(void);
  * max_nodes[1] on 256 (4 per CTA), up to max_nodes[2] on 512 (2 per CTA),
  * larger ones on 1024 threads.  A call with too few instances to fill the GPU
  * with teams of that width takes wider ones.  The potentials do not depend on
- * the team, the LP value only through the order of its team-wide sum (~1e-16
- * relative).  f2m_b200/autotune.py times candidate bounds
+ * the team, and the LP value, a sum in the order of the team that the size asks
+ * for, only on the bounds (~1e-16 relative); a single instance that runs on the
+ * whole GPU sums in another order.  f2m_b200/autotune.py times candidate bounds
  * on a workload.  The bounds are process-wide: set them before solving.
- * F2M_ERR_INPUT if not
- * increasing or a class's shared memory cannot hold an instance that size. */
+ * F2M_ERR_INPUT if not increasing or a class's shared memory cannot hold an
+ * instance that size. */
 f2m_status f2m_set_class_bounds(const int32_t* max_nodes); /* 3 values */
 void f2m_get_class_bounds(int32_t* max_nodes);
 /* Shared memory a CTA of the batched solver takes, in KB (no reference

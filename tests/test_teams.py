@@ -55,3 +55,15 @@ def test_potentials_equal_the_oracles_on_every_team(ctx, instances, per_sm, narr
         # (an instance whose irregular combs went through the repair loop holds the
         # potentials of its last step, as the oracle's)
         assert np.array_equal(F[offs[i]:offs[i] + o.n_nodes], o.F), len(instances[0][i][0])
+
+
+def test_lp_bits_do_not_depend_on_the_call(ctx, instances):
+    """The LP value sums in the order of the team that the size asks for."""
+    lps = []
+    for per_sm in (0.5, 1.5, 3, 5, 9):
+        offs, x, y = _call(instances, int(per_sm * _sms()))
+        lps.append(ctx.solve_batch(offs, x, y, N)[0][:len(instances[0])])
+    for lp in lps[1:]:
+        assert np.array_equal(lp, lps[0], equal_nan=True)
+    for i, (x, y) in enumerate(instances[0]):
+        assert ctx.solve_batch(np.array([0, len(x)]), x, y, N)[0][0] == lps[0][i]
