@@ -727,24 +727,40 @@ __device__ __forceinline__ void primal_node(const Batch& B, const Inst& I, HP H,
     ps.fsum += 2.0 * hv;
     float degsum = 0.0f;
     bool any = false;
-    for (int64_t a = r0; a < r1; ++a) {
-        const Slot s = I.slot[a];
-        const double d = red_d(s, v, H, hv);
-        double x = (d < porog) ? ((d > -porog) ? 0.5 : 1.0) : 0.0;
-        uint8_t code = (uint8_t)(x == 1.0 ? 2 : (x == 0.5 ? 1 : 0));
-        if (axb && code == 1) {
-            const int l1 = lab[v], l2 = lab[s.nbr];
-            const int c = (l2 == INT_MAX) ? l1 : (l1 == INT_MAX ? l2 : ::max(l1, l2));
-            if (c != INT_MAX && irr[c]) { x = (double)B.xval[a]; code = 3; }
+    // (four slots' loads ahead of the stores of their codes, which may alias anything)
+    for (int64_t a0 = r0; a0 < r1; a0 += 4) {
+        Slot sl[4];
+        double cost[4];
+        int mir[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t a = a0 + i < r1 ? a0 + i : r1 - 1;
+            sl[i] = I.slot[a];
+            cost[i] = B.s_cost[a];
+            mir[i] = B.mirror[a];
         }
-        B.xcode[a] = code;
-        const bool in_x = (x != 0.0) || code == 3;
-        degsum += (float)x;
-        any |= in_x;
-        if (s.nbr > v) {
-            ps.lp += x * B.s_cost[a];
-            ps.dual_neg += fmin(0.0, d);
-            if (in_x) ps.maxr = ::max(ps.maxr, (long long)::min((int)(a - r0), B.mirror[a]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t a = a0 + i;
+            if (a >= r1) break;
+            const Slot s = sl[i];
+            const double d = red_d(s, v, H, hv);
+            double x = (d < porog) ? ((d > -porog) ? 0.5 : 1.0) : 0.0;
+            uint8_t code = (uint8_t)(x == 1.0 ? 2 : (x == 0.5 ? 1 : 0));
+            if (axb && code == 1) {
+                const int l1 = lab[v], l2 = lab[s.nbr];
+                const int c = (l2 == INT_MAX) ? l1 : (l1 == INT_MAX ? l2 : ::max(l1, l2));
+                if (c != INT_MAX && irr[c]) { x = (double)B.xval[a]; code = 3; }
+            }
+            B.xcode[a] = code;
+            const bool in_x = (x != 0.0) || code == 3;
+            degsum += (float)x;
+            any |= in_x;
+            if (s.nbr > v) {
+                ps.lp += x * cost[i];
+                ps.dual_neg += fmin(0.0, d);
+                if (in_x) ps.maxr = ::max(ps.maxr, (long long)::min((int)(a - r0), mir[i]));
+            }
         }
     }
     if (any && !(degsum > 2.0f - 1e-2f && degsum < 2.0f + 1e-2f)) ps.viol++;
