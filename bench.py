@@ -587,17 +587,15 @@ def smooth_sub(args, local_rank, steps=3, warmup=1):
         t0 = time.perf_counter()
         L, gx, gy = ctx.smoothed_bound(offs, x, y, N, params=p, grad=True)
         ms.append(1e3 * (time.perf_counter() - t0))
-        tr, km = ctx.smooth_work()  # logistic terms and time of the persistent kernel
-        kterms.append(tr)
+        _, km = ctx.smooth_work()  # time of the persistent kernel
+        kterms.append(ctx.smooth_taken())  # and the logistic terms it evaluated
         kms.append(km)
     clocks = clk.stop()
     launches = ctx.kernel_launches() - l0
-    # the persistent kernel's rate of logistic terms (one FP64 exp and one
-    # division each: the Newton sums of every node root, softplus, sigma and
-    # sigma') beside the rate of evaluating each of them, measured at full
-    # occupancy on this GPU.  The sums cover every list entry; entries out of
-    # reach of the root are counted and not evaluated, so the ratio is no
-    # fraction of a peak and may pass 1.
+    # the persistent kernel's rate of logistic terms evaluated (one FP64 exp and
+    # one division each: entries within reach in the Newton sums of every node
+    # root and in the reverse passes, softplus, sigma) against the rate of that
+    # term measured at full occupancy on this GPU
     peak_terms = ctx.fp64_rate(2, repeats=3)
     ctx.close()
     t = float(np.mean(ms))
@@ -620,8 +618,7 @@ def smooth_sub(args, local_rank, steps=3, warmup=1):
                      "peak_kind": "measured in this run (f2m_fp64_rate kind 2: the same term, four "
                                   "independent sums per thread, every SM at full occupancy)",
                      "terms_per_launch": float(np.mean(kterms)), "kernel_ms": float(np.mean(kms)),
-                     "terms": "list entries the sums cover; those out of reach of the root are "
-                              "counted and not evaluated",
+                     "terms": "list entries within reach of a root: those evaluated",
                      "traffic": None},
     }
     if not args.no_cpu_baseline:
@@ -754,8 +751,8 @@ def smooth_arm(args, rank, world, local_rank):
         t0 = time.perf_counter()
         L, gx, gy = ctx.smoothed_bound(offs, x, y, N, params=p, grad=True)
         ms.append(1e3 * (time.perf_counter() - t0))
-        tr, km = ctx.smooth_work()
-        kterms.append(tr)
+        _, km = ctx.smooth_work()
+        kterms.append(ctx.smooth_taken())
         kms.append(km)
     clocks = clk.stop()
     launches = ctx.kernel_launches() - l0

@@ -94,7 +94,7 @@ EXPORTS = [
     "f2m_get_class_bounds", "f2m_solve_graph", "f2m_solve_points_from", "f2m_fp64_rate",
     "f2m_partition_selfcheck", "f2m_smooth_work",
     "f2m_smoothed_bound_bwd_edges", "f2m_set_solver_smem_kb", "f2m_get_solver_smem_kb",
-    "f2m_batch_potentials", "f2m_team_width",
+    "f2m_batch_potentials", "f2m_team_width", "f2m_smooth_taken",
 ]
 
 _lib = None
@@ -142,6 +142,7 @@ def lib():
         L.f2m_fp64_rate.argtypes = [vp, i32, i32, P(dbl)]
         L.f2m_partition_selfcheck.argtypes = [vp, i32, ctypes.c_uint64, P(ctypes.c_int64)]
         L.f2m_smooth_work.argtypes = [vp, P(ctypes.c_int64), P(ctypes.c_float)]
+        L.f2m_smooth_taken.argtypes = [vp, P(ctypes.c_int64)]
         L.f2m_solve_points_noalloc.argtypes = [vp, vp, i32, i32, P(Params), vp, vp, vp]
         L.f2m_default_smooth_params.argtypes = [P(SmoothParams)]
         L.f2m_smoothed_bound_fwd.argtypes = [vp, i32, vp, vp, vp, i32, P(SmoothParams), vp]
@@ -329,6 +330,13 @@ class Context:
         ms = ctypes.c_float()
         self._check(lib().f2m_smooth_work(self._h, ctypes.byref(t), ctypes.byref(ms)))
         return t.value, ms.value
+
+    def smooth_taken(self):
+        """Logistic terms that the last smoothed-bound call's persistent kernel
+        evaluated (entries within reach of a root); -1 after the per-step path."""
+        t = ctypes.c_int64()
+        self._check(lib().f2m_smooth_taken(self._h, ctypes.byref(t)))
+        return t.value
 
     def partition_selfcheck(self, n_cases=100000, seed=1):
         """Lists on which the warp-cooperative partition and the serial one

@@ -305,7 +305,7 @@ struct SmoothBatch {
     float* gx = nullptr;                // [n_total]
     float* gy = nullptr;                // [n_total]
     int32_t* queue = nullptr;
-    unsigned long long* work = nullptr; // [1] logistic terms covered by the persistent kernel
+    unsigned long long* work = nullptr; // [2] logistic terms covered and taken by the persistent kernel
 };
 cudaError_t launch_smooth_graph(SmoothBatch& S, int64_t* scan_scratch, cudaStream_t s,
                                 int64_t* launches);

@@ -79,7 +79,7 @@ struct f2m_ctx {
     std::vector<int64_t> skey;
     int64_t sgraph_launches = 0;
     // work and kernel time of the last smoothed-bound call (persistent path)
-    int64_t smooth_terms = -1;
+    int64_t smooth_terms = -1, smooth_taken = -1;
     float smooth_ms = 0.f;
 };
 
@@ -1372,6 +1372,11 @@ f2m_status f2m_smooth_work(const f2m_ctx* ctx, int64_t* terms, float* kernel_ms)
     if (kernel_ms) *kernel_ms = ctx->smooth_ms;
     return F2M_OK;
 }
+f2m_status f2m_smooth_taken(const f2m_ctx* ctx, int64_t* terms) {
+    if (!ctx || !terms) return F2M_ERR_INPUT;
+    *terms = ctx->smooth_taken;
+    return F2M_OK;
+}
 
 f2m_status f2m_partition_selfcheck(f2m_ctx* ctx, int32_t n_cases, uint64_t seed, int64_t* mismatches) {
     if (!ctx || !mismatches || n_cases < 0)
@@ -2138,7 +2143,7 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
         B.L = A.take<double>(n_inst);
         dLd = A.take<double>(n_inst);
         B.queue = A.take<int32_t>(1);
-        B.work = A.take<unsigned long long>(1);
+        B.work = A.take<unsigned long long>(2);
         if (q.steps) {
             B.ua = A.take<double>(n);
             B.ub = A.take<double>(n);
@@ -2224,7 +2229,7 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
                              cudaMemcpyHostToDevice, ctx->stream));
     F2M_CUDA(launch_smooth_entries(B, ctx->stream, &ctx->launches));
     B.solver = steps ? 2 : 1;
-    ctx->smooth_terms = -1;
+    ctx->smooth_terms = ctx->smooth_taken = -1;
     ctx->smooth_ms = 0.f;
     if (steps) {
         F2M_CUDA(smooth_steps_graph(ctx, B, grad));
@@ -2236,11 +2241,12 @@ f2m_status smooth_call(f2m_ctx* ctx, int32_t n_inst, const int64_t* offs, const 
     F2M_CUDA(cudaMemcpyAsync(L, B.L, n_inst * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     if (gx) F2M_CUDA(cudaMemcpyAsync(gx, B.gx, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     if (gy) F2M_CUDA(cudaMemcpyAsync(gy, B.gy, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    unsigned long long terms = 0;
-    if (!steps) F2M_CUDA(cudaMemcpyAsync(&terms, B.work, sizeof(terms), cudaMemcpyDeviceToHost, ctx->stream));
+    unsigned long long terms[2] = {0, 0};
+    if (!steps) F2M_CUDA(cudaMemcpyAsync(terms, B.work, sizeof(terms), cudaMemcpyDeviceToHost, ctx->stream));
     F2M_CUDA(cudaStreamSynchronize(ctx->stream));
     if (!steps) {
-        ctx->smooth_terms = (int64_t)terms;
+        ctx->smooth_terms = (int64_t)terms[0];
+        ctx->smooth_taken = (int64_t)terms[1];
         F2M_CUDA(cudaEventElapsedTime(&ctx->smooth_ms, ctx->ev[0], ctx->ev[1]));
     }
     if (eo && grad) {

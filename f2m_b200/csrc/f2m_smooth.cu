@@ -520,11 +520,16 @@ __device__ __forceinline__ void warp_ord_max(double x, long long* slot) {
     if ((threadIdx.x & 31) == 0) atomicMax(slot, ord_of(x));
 }
 
+// Terms of the sums: list entries they cover, and those taken (an exponential
+// each; the others are out of reach).
+struct STerms {
+    unsigned long long covered = 0, taken = 0;
+};
 // The root of a node given the potentials u and a bound umax >= every u; *thr
-// receives m2 + kReach tau.  terms counts the list terms the sums cover.
+// receives m2 + kReach tau.
 template <int G, class List, class UP>
 __device__ __forceinline__ double node_root(const SmoothBatch& S, const List& L, UP u, double umax, const SBuf& B,
-                                            double* thr, unsigned long long& terms) {
+                                            double* thr, STerms& terms) {
     constexpr int C = G >= 8 ? 2 : 4;  // columns read at once
     const bool lead = threadIdx.x % G == 0;
     const double win = kReach * S.tau;
@@ -558,7 +563,8 @@ __device__ __forceinline__ double node_root(const SmoothBatch& S, const List& L,
     for (int it = 0; it < S.newton_max; ++it) {
         LogitAcc r;
         if (go) {
-            if (lead) terms += (unsigned long long)L.deg;
+            if (lead) terms.covered += L.deg;
+            terms.taken += cnt;
             if (cnt <= B.cap) {
                 #pragma unroll 2
                 for (int j = 0; j < cnt; ++j) r.add((s - B.x[j * B.stride]) * S.inv_tau);
@@ -598,7 +604,7 @@ __device__ __forceinline__ double node_root(const SmoothBatch& S, const List& L,
 // q_e = mu_v p_e added to the node's share of dL/dc.
 template <int G, class List, class UP>
 __device__ __forceinline__ double node_rev1(const SmoothBatch& S, const List& L, UP u, double umax, const SBuf& B,
-                                            double s, double thr, double lam, unsigned long long& terms) {
+                                            double s, double thr, double lam, STerms& terms) {
     constexpr int C = G >= 8 ? 2 : 4;
     int cnt = 0, end = 0;
     while (end < L.n) {
@@ -613,7 +619,8 @@ __device__ __forceinline__ double node_rev1(const SmoothBatch& S, const List& L,
         end = min(end + C, L.n);
         if ((double)__uint_as_float(e[C - 1].x) - umax > thr) break;
     }
-    if (threadIdx.x % G == 0) terms += (unsigned long long)L.deg;
+    if (threadIdx.x % G == 0) terms.covered += L.deg;
+    terms.taken += cnt;
     double D = 0.0;
     auto p_of = [&](double a) { return dsig((s - a) * S.inv_tau) * S.inv_tau; };
     auto each = [&](auto f) {  // entries within reach, re-read
@@ -647,7 +654,7 @@ __device__ __forceinline__ double node_rev1(const SmoothBatch& S, const List& L,
 // formed from the same operands as in pass 1, so q need not be stored.
 template <int G, class List, class TP, class SP, class MP>
 __device__ __forceinline__ double node_rev2(const SmoothBatch& S, const List& L, double uw, double thrmax, TP thr,
-                                            SP s, MP mu, const SBuf& B) {
+                                            SP s, MP mu, const SBuf& B, STerms& terms) {
     constexpr int C = G >= 8 ? 2 : 4;
     int cnt = 0, end = 0;
     while (end < L.n) {
@@ -662,6 +669,7 @@ __device__ __forceinline__ double node_rev2(const SmoothBatch& S, const List& L,
         end = min(end + C, L.n);
         if ((double)__uint_as_float(e[C - 1].x) - uw > thrmax) break;
     }
+    terms.taken += cnt;
     double sum = 0.0;
     auto q_of = [&](int v, double a) { return mu[v] * (dsig((s[v] - a) * S.inv_tau) * S.inv_tau); };
     if (cnt <= B.cap) {
@@ -683,7 +691,7 @@ __device__ __forceinline__ double node_rev2(const SmoothBatch& S, const List& L,
 // given, and the largest new potential into *umax_next.
 __device__ __forceinline__ void sjacobi(const SmoothBatch& S, const SInst& I, const double* u, double* un,
                                         double* s_out, double* t_out, const SBuf& B, double umax,
-                                        long long* umax_next, unsigned long long& terms) {
+                                        long long* umax_next, STerms& terms) {
     double mx = -INFINITY;
     const int v1 = (I.V + 31) & ~31;  // whole warps
     for (int v = threadIdx.x; v < v1; v += kST) {
@@ -702,13 +710,13 @@ __device__ __forceinline__ void sjacobi(const SmoothBatch& S, const SInst& I, co
 }
 
 __device__ double sbound(const SmoothBatch& S, const SInst& I, const double* u, double* sred,
-                         unsigned long long& terms) {
+                         STerms& terms) {
     double su = 0.0, sp = 0.0;
     for (int v = threadIdx.x; v < I.V; v += kST) {
         su += 2.0 * u[v];
         for (int64_t k = I.row[v]; k < I.row[v + 1]; ++k) {
             const int w = S.nbr[k];
-            if (w > v) { sp += softplus((u[v] + u[w] - (double)S.c[k]) / S.tau); ++terms; }
+            if (w > v) { sp += softplus((u[v] + u[w] - (double)S.c[k]) / S.tau); ++terms.covered; ++terms.taken; }
         }
     }
     su = block_sum<kST>(su, sred);
@@ -732,16 +740,19 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
     double* Ha = reinterpret_cast<double*>(smem_raw);
     double* bx = Ha + 2 * (size_t)max_v;
     const SBuf B{bx + threadIdx.x, reinterpret_cast<uint16_t*>(bx + (size_t)cap * kST) + threadIdx.x, kST, cap};
-    // list terms the sums of this thread cover (Newton sums, softplus, sigma,
+    // terms of this thread's sums (Newton sums, softplus, sigma,
     // sigma'), added to S.work when the queue is empty
-    unsigned long long terms = 0;
+    STerms terms;
     for (;;) {
         if (threadIdx.x == 0) sitem = atomicAdd(S.queue, 1);
         __syncthreads();
         const int item = sitem;
         __syncthreads();
         if (item >= S.n_inst) {
-            if (S.work && terms) atomicAdd(S.work, terms);
+            if (S.work) {
+                if (terms.covered) atomicAdd(S.work, terms.covered);
+                if (terms.taken) atomicAdd(S.work + 1, terms.taken);
+            }
             return;
         }
         SInst I;
@@ -782,7 +793,8 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
                 const double z = (u[v] + u[S.nbr[k]] - (double)S.c[k]) / S.tau;
                 r.add(z);
                 S.gc[k] = up * (0.5 * sigm(z));
-                terms += 2;
+                terms.covered += 2;
+                terms.taken += 2;
             }
             lam[v] = up * (-((r.cnt - 2.0) + r.tail));  // 2 - sum sigma
         }
@@ -847,7 +859,7 @@ __global__ void __launch_bounds__(kST, 2) k_sbound(SmoothBatch S, int cap, int m
                     const bool in = v < I.V;
                     const auto nd = slice_part(S, I, v, in);
                     const double x = node_rev2<1>(S, nd, in ? Ha[v] : 0.0, thrmax, (const double*)Hb, st,
-                                                    (const double*)mu, B);
+                                                    (const double*)mu, B, terms);
                     if (in) lam2[v] = (1.0 - S.omega) * lam[v] - x;
                     __syncwarp();
                 }
@@ -897,7 +909,7 @@ __global__ void __launch_bounds__(kWT) k_sw_step(SmoothBatch S, const double* u,
     SThread<kWG> t;
     if (!step_thread(S, t)) return;
     double mx = -INFINITY, thr;
-    unsigned long long terms = 0;
+    STerms terms;
     const double s = node_root<kWG>(S, t.nd, u + t.base, ord_to(umax[t.b]), B, &thr, terms);
     if (t.lead) {
         const int64_t g = t.g;
@@ -997,7 +1009,7 @@ __global__ void __launch_bounds__(kWT) k_sw_rev1(SmoothBatch S, const double* ut
     F2M_SBUF;
     SThread<kWG> t;
     if (!step_thread(S, t)) return;
-    unsigned long long terms = 0;
+    STerms terms;
     const double thr = t.in ? tv[t.g] : -INFINITY;
     const double mu = node_rev1<kWG>(S, t.nd, ut + t.base, ord_to(umax[t.b]), B, t.in ? st[t.g] : 0.0, thr,
                                      t.in ? lam[t.g] : 0.0, terms);
@@ -1012,8 +1024,9 @@ __global__ void __launch_bounds__(kWT) k_sw_rev2(SmoothBatch S, const double* ut
     F2M_SBUF;
     SThread<kWG> t;
     if (!step_thread(S, t)) return;
+    STerms terms;
     const double x = node_rev2<kWG>(S, t.nd, t.in ? ut[t.g] : 0.0, ord_to(thrmax[t.b]), tv + t.base, st + t.base,
-                                    (const double*)S.mu + t.base, B);
+                                    (const double*)S.mu + t.base, B, terms);
     if (t.lead) lam2[t.g] = (1.0 - S.omega) * lam[t.g] - x;
 }
 
@@ -1254,7 +1267,7 @@ cudaError_t launch_smooth_bound(SmoothBatch& S, int32_t max_v, bool grad, cudaSt
     int grid = sms * per_sm;
     if (grid > S.n_inst) grid = S.n_inst;
     if ((e = cudaMemsetAsync(S.queue, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
-    if (S.work && (e = cudaMemsetAsync(S.work, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    if (S.work && (e = cudaMemsetAsync(S.work, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
     if (grad && (e = clear_smooth_sums(S, s)) != cudaSuccess) return e;
     if (grad) k_sbound<true><<<grid, kST, dyn, s>>>(S, cap, max_v);
     else k_sbound<false><<<grid, kST, dyn, s>>>(S, cap, max_v);

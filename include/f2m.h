@@ -175,6 +175,9 @@ f2m_status f2m_partition_selfcheck(f2m_ctx* ctx, int32_t n_cases, uint64_t seed,
  * are counted, not evaluated -- and that kernel's CUDA-event time in ms.
  * terms is -1 when the call took the one-launch-per-step path. */
 f2m_status f2m_smooth_work(const f2m_ctx* ctx, int64_t* terms, float* kernel_ms);
+/* Of those, and of the reverse steps' second passes, the terms that were within
+ * reach and so evaluated (an FP64 exponential each); -1 likewise. */
+f2m_status f2m_smooth_taken(const f2m_ctx* ctx, int64_t* terms);
 
 /* ------------------------------------------------------------------ */
 /* Single instance with full results (the F2M.h graph API).             */

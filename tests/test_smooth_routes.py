@@ -82,3 +82,20 @@ def test_steps_over_many_points(ctx, oracle, make, N, tau):
     assert offs[-1] > 14000
     _check(ctx, oracle, offs, x, y, N, tau, 20, 2, (0, 1, 2, 3, 4, 5, 6, 8, 10, len(sizes) - 1))
     _check(ctx, oracle, offs, x, y, N, tau, 20, 1, (0, 4, 7, len(sizes) - 1))
+
+
+def test_terms_taken_are_those_within_reach(ctx):
+    """Cold lattices have three or four of some 36 entries within reach; at a warm
+    temperature whole lists are, and the reverse steps' second passes come on top."""
+    offs, x, y = _batch(synth.jittered_lattice, [400, 500, 600], 40)
+    taken = {}
+    for tau in (1e-3, 0.5):
+        p = f2m_b200.default_smooth_params(tau=tau, iters=10, solver=1)
+        for grad in (False, True):
+            ctx.smoothed_bound(offs, x, y, 24, params=p, grad=grad)
+            taken[tau, grad] = ctx.smooth_taken() / ctx.smooth_work()[0]
+    # (the bound itself takes every edge once, less than a tenth of what ten steps cover)
+    assert 3 / 48 < taken[1e-3, False] < 0.25 and 3 / 48 < taken[1e-3, True] < 0.25
+    assert taken[0.5, False] == 1.0 and taken[0.5, True] > 1.0
+    ctx.smoothed_bound(offs, x, y, 24, params=f2m_b200.default_smooth_params(solver=2))
+    assert ctx.smooth_taken() == -1
