@@ -864,8 +864,8 @@ struct Team {
 //
 // While the lists stand, the potentials are kept in slice order too (position
 // 32*s + l; the words hold positions): a lane's own potential is then read and
-// written with unit stride, where node order costs about six wavefronts for
-// each of the two.  The places past V in the last slice repeat its first node,
+// written with unit stride, where node order costs a gather for each of the
+// two.  The places past V in the last slice repeat its first node,
 // list included, so no lane is an exception.  Partitions and combs use node
 // order (to_nodes); an instance with a node-indexed slice stays in it.
 struct TeamMem {
@@ -1057,12 +1057,12 @@ __device__ __forceinline__ void step_barrier(int bar, int threads) {
 // n Jacobi steps over fixed lists by warp w of the team, w < min(NS, warps),
 // whose slices are w, w + warps, ... (longest lists first).  A step is a short
 // dependent chain: a gather, two additions, the selection, a store and a
-// barrier.  On a full SM the shared-memory gathers bound it (a random 8-byte
-// gather takes about six wavefronts), so what does not change between
-// rebuilds -- D, the neighbours' offsets, the order flags and the own
-// potential, which only this lane writes -- stays in registers where it can.
-// A slice of three entries then takes 20 cycles of an SM; read from the SELL
-// arrays it takes about 35 in shared memory and 60 through L1 and L2.
+// barrier.  On a full SM the loads bound it, the gathers with their bank conflicts
+// first, so what does not change between rebuilds -- D, the neighbours' offsets,
+// the order flags and the own potential, which only this lane writes -- stays in
+// registers where it can.  (4,096 instances of 50-5,000 points, solve phase: 144
+// ms with every list in the SELL arrays and node order, 107 so, the selection
+// networks included.)
 //
 // step_one: the warp's only slice, of width <= K, in registers.
 template <int K>
@@ -1096,9 +1096,8 @@ __device__ __noinline__ void step_one(StepView M, int w, int lane, int n) {
 // step_slices: the last R slices, of width <= 3, in registers (16-bit byte
 // offsets, two to a register, so V <= 8,160), and with HEAD the first slice, of
 // width <= HEAD; with MEM the warp's other slices come from the SELL arrays.
-// (The few warps whose first slice is wider set the pace of a step: 96 slices
-// on 32 warps take 2,060 cycles when all are three wide, 4,020 with twelve
-// four-wide heads read from the SELL arrays.)
+// (The few warps whose first slice is wider set the pace of a step, so heads of up
+// to eight entries are kept in registers too.)
 constexpr int kPackedMaxV = 8160;
 template <int R, int HEAD, bool MEM>
 __device__ __noinline__ void step_slices(StepView M, int w, int lane, int n) {
@@ -1874,8 +1873,10 @@ int solve_team_width(int c) { return kClasses[c].team; }
 // GPU; a call with fewer instances than that leaves SMs idle, and a solve is
 // thousands of dependent steps, so each instance then gets the most threads it
 // can have: a call of up to 148 instances runs on 1,024-thread teams, one to an
-// SM (64 instances of 50-320 points 8.7 -> 4.4 ms with it, one of 300 points
-// 3.4 -> 2.6 ms, against the 128-thread teams their size asks for).
+// SM.  Solve phase on the team that the size asks for / on the widest resident:
+// 64 instances of 50-320 points 2.5 / 1.3 ms, of 500-1,200 15.4 / 12.3; 220 of
+// 50-320 3.8 / 1.8, of 250-440 7.3 / 2.7, of 500-1,200 18.3 / 16.7, of 900-1,700
+// 18.2 / 18.0; 450 of 250-440 7.6 / 4.8, of 500-1,200 21.9 / 21.3.
 int solve_wide_class(int64_t n_inst) {
     int dev = 0, sms = 0, wide = 0;
     cudaGetDevice(&dev);

@@ -791,7 +791,10 @@ void carve_edge_sort(Arena& A, EdgeSort& E, int64_t S) {
 // SM could hold it: its 148 CTAs exchange potentials every few steps, but share
 // the work of a step.  Solve phase on one SM / on all: 1,000 points 1.7 / 2.8
 // ms, 2,000 points 4.8 / 4.6, 3,000 points 14.0 / 11.3, 5,000 points 20.8 / 6.3,
-// 8,000 points 33.3 / 7.0.  Without coordinates (f2m_solve_graph) the CTAs' halos
+// 8,000 points 33.3 / 7.0.  Calls on several contexts then take turns: 1 / 4 / 16
+// threads with one each, ms a call, 3,000 points 12.6 / 11.6 / 11.5 (on one SM each
+// 15.6 / 4.2 / 2.9), 5,000 points 7.7 / 6.6 / 6.5 (23.1 / 6.0 / 5.8), 8,000 points
+// 8.8 / 7.7 / 7.2 (36.1 / 9.4 / 7.6).  Without coordinates (f2m_solve_graph) the CTAs' halos
 // are not local, so those keep the one SM.
 constexpr int32_t kGridSingle = 2500;
 bool takes_grid(int32_t n, int32_t n_inst, const f2m_params& prm, bool spatial) {

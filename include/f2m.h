@@ -60,8 +60,10 @@ typedef struct f2m_params {
     int32_t solver;        /* 0 auto: a team per instance; a single instance above 2,500 points
                               (10,000 from f2m_solve_graph; distinct points count) takes the
                               whole GPU;
-                              1: a team up to 10,000 points (one SM: for callers that run many
-                              single solves side by side, on a context per thread);
+                              1: a team up to 10,000 points (one SM: several single solves
+                              run side by side, on a context per thread, where those on the
+                              whole GPU take turns: from about four threads on this is the
+                              faster way up to 5,000 points);
                               2: the whole-GPU solver for a single instance of any size */
     int64_t grid_spin_limit; /* the whole-GPU solver's grid barrier is a bounded wait: after
                               this many polls a CTA gives up, every CTA leaves the solve and
