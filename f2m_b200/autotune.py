@@ -3,7 +3,9 @@
 The batched solver runs each instance on a team of 128, 256, 512 or 1024
 threads (8, 4, 2 or 1 teams per CTA) chosen by its point count; the three
 bounds between the classes decide how shared memory and SMs are split
-across a batch of uneven instances, and the shared memory a CTA takes
+across a batch of uneven instances (calls with too few instances to fill the
+GPU take wider teams whatever the bounds: tune on more than eight an SM), and the
+shared memory a CTA takes
 decides how much of each SM stays L1 cache for the list slices that spill
 to global memory.  The potentials never depend on either (the LP value only
 through the order of a sum).  This script times the solve phase (CUDA

@@ -38,8 +38,8 @@ def _check(ctx, oracle, offs, x, y, N, tau, iters, solver, sample):
         # compared where the oracle has a value
         fx, fy = np.isfinite(dx), np.isfinite(dy)
         scale = max(np.abs(dx[fx]).max(), np.abs(dy[fy]).max())
-        assert np.abs(gx[s] - dx)[fx].max() <= 1e-5 * scale
-        assert np.abs(gy[s] - dy)[fy].max() <= 1e-5 * scale
+        assert np.abs(gx[s][fx] - dx[fx]).max() <= 1e-5 * scale
+        assert np.abs(gy[s][fy] - dy[fy]).max() <= 1e-5 * scale
 
 
 def _many():
